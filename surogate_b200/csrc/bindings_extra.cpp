@@ -333,7 +333,7 @@ std::vector<Tensor> nvfp4_quantize(const Tensor& x, const Tensor& amax, bool sto
     TORCH_CHECK(K % 16 == 0 && (!block2d || rows % 16 == 0), "nvfp4_quantize: K (and rows for 2-D blocks) must be multiples of 16");
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor q = torch::empty({rows, K / 2}, x.options().dtype(at::kByte));
-    Tensor sf = torch::zeros({nvfp4_sf_bytes(rows, K)}, x.options().dtype(at::kByte));
+    Tensor sf = torch::empty({nvfp4_sf_bytes(rows, K)}, x.options().dtype(at::kByte));   // the kernel writes the padding too
     sg_count_launch(1);
     sg::nvfp4_quantize_rows(x.data_ptr(), q.data_ptr(), sf.data_ptr(), amax.data_ptr<float>(), rows, K, stochastic, static_cast<uint32_t>(seed), block2d,
                             sms(), cur_stream(), four_over_six && !stochastic);
@@ -348,7 +348,7 @@ std::vector<Tensor> nvfp4_quantize_transpose(const Tensor& x, const Tensor& amax
     TORCH_CHECK(R % 64 == 0 && C % 64 == 0, "nvfp4_quantize_transpose: both dimensions must be multiples of 64");
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor q = torch::empty({C, R / 2}, x.options().dtype(at::kByte));
-    Tensor sf = torch::zeros({nvfp4_sf_bytes(C, R)}, x.options().dtype(at::kByte));
+    Tensor sf = torch::empty({nvfp4_sf_bytes(C, R)}, x.options().dtype(at::kByte));
     sg_count_launch(1);
     sg::nvfp4_quantize_transpose(x.data_ptr(), q.data_ptr(), sf.data_ptr(), amax.data_ptr<float>(), R, C, stochastic, hadamard,
                                  static_cast<uint32_t>(seed), static_cast<uint32_t>(sign_mask), cur_stream(), four_over_six && !stochastic);

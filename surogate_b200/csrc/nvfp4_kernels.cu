@@ -16,6 +16,7 @@
 //
 // Replaces recipes/nvfp4/kernels/{quant_fp4,quant_nvfp4_cutlass,hadamard}.cu of the reference.
 #include <cuda_bf16.h>
+#include <cuda_fp4.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -40,38 +41,31 @@ __device__ __forceinline__ float hash_uniform(uint32_t seed, uint64_t idx) {
     return static_cast<float>(static_cast<uint32_t>(z >> 40)) * (1.0f / 16777216.0f);
 }
 
-// e2m1 code (4 bits: sign | 3-bit magnitude index into {0, .5, 1, 1.5, 2, 3, 4, 6}), round-to-nearest-even on the grid
-__device__ __forceinline__ uint32_t e2m1_rn(float v) {
-    const uint32_t sign = v < 0.f ? 8u : 0u;
-    const float a = fminf(fabsf(v), 6.f);
-    uint32_t code;
-    if (a <= 0.25f) code = 0;
-    else if (a < 0.75f) code = 1;
-    else if (a <= 1.25f) code = 2;
-    else if (a < 1.75f) code = 3;
-    else if (a <= 2.5f) code = 4;
-    else if (a < 3.5f) code = 5;
-    else if (a <= 5.0f) code = 6;
-    else code = 7;
-    return sign | code;
+// two e2m1 codes (4 bits: sign | 3-bit magnitude index into {0, .5, 1, 1.5, 2, 3, 4, 6}) in one byte, low nibble first; round to
+// nearest even on the grid, saturating: one conversion instruction per pair instead of a chain of seven compares per element.
+// The addition turns -0 into +0, so that a zero always has code 0.
+__device__ __forceinline__ uint32_t e2m1x2_rn(float lo, float hi) {
+    return __nv_cvt_float2_to_fp4x2(make_float2(lo + 0.f, hi + 0.f), __NV_E2M1, cudaRoundNearest);
+}
+__device__ __forceinline__ float2 e2m1x2_value(uint32_t codes) {
+    return __half22float2(__half2(__nv_cvt_fp4x2_to_halfraw2(static_cast<__nv_fp4x2_storage_t>(codes), __NV_E2M1)));
 }
 __device__ __forceinline__ float e2m1_value(uint32_t code) {
     const float mag[8] = {0.f, 0.5f, 1.f, 1.5f, 2.f, 3.f, 4.f, 6.f};
     const float m = mag[code & 7];
     return (code & 8) ? -m : m;
 }
-// stochastic rounding between the two neighbouring grid points (unbiased for |v| <= 6)
+// stochastic rounding between the two neighbouring grid points (unbiased for |v| <= 6).  From 1 upwards the grid is the floats with
+// one mantissa bit, so the lower neighbour is a truncation and its code a shift; below 1 it is 0 or 0.5.
 __device__ __forceinline__ uint32_t e2m1_sr(float v, float u) {
     const uint32_t sign = v < 0.f ? 8u : 0u;
     const float a = fminf(fabsf(v), 6.f);
-    const float grid[8] = {0.f, 0.5f, 1.f, 1.5f, 2.f, 3.f, 4.f, 6.f};
-    int lo = 0;
-#pragma unroll
-    for (int i = 1; i < 8; ++i)
-        if (a >= grid[i]) lo = i;
-    if (lo == 7) return sign | 7u;
-    const float p = (a - grid[lo]) / (grid[lo + 1] - grid[lo]);
-    return sign | static_cast<uint32_t>(u < p ? lo + 1 : lo);
+    const uint32_t bits = __float_as_uint(a);
+    const bool big = a >= 1.f, half = a >= 0.5f;
+    const uint32_t lo = big ? (bits >> 22) - 252u : (half ? 1u : 0u);
+    const float base = big ? __uint_as_float(bits & 0xFFC00000u) : (half ? 0.5f : 0.f);
+    const float inv_gap = big ? __uint_as_float((255u << 23) - (bits & 0x7F800000u)) : 2.f;   // 1 / (2^e / 2)
+    return sign | (lo + (u < (a - base) * inv_gap ? 1u : 0u));                                  // a = 6 has no remainder: stays code 7
 }
 
 __device__ __forceinline__ float decode_e4m3(uint8_t b) {
@@ -94,10 +88,10 @@ __device__ __forceinline__ uint8_t quant_block16(const float (&v)[16], float ge,
     const float mul = sfd > 0.f ? ge / sfd : 0.f;
     out[0] = out[1] = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float s = v[i] * mul;
-        const uint32_t c = SR ? e2m1_sr(s, hash_uniform(seed, base_idx + i)) : e2m1_rn(s);
-        out[i >> 3] |= c << ((i & 7) * 4);   // element 2j in the low nibble of byte j
+    for (int i = 0; i < 16; i += 2) {      // element 2j in the low nibble of byte j
+        const float s0 = v[i] * mul, s1 = v[i + 1] * mul;
+        const uint32_t c = SR ? e2m1_sr(s0, hash_uniform(seed, base_idx + i)) | (e2m1_sr(s1, hash_uniform(seed, base_idx + i + 1)) << 4) : e2m1x2_rn(s0, s1);
+        out[i >> 3] |= c << ((i & 7) * 4);
     }
     return sfb;
 }
@@ -125,11 +119,13 @@ __device__ __forceinline__ uint8_t quant_block16_4o6(const float (&v)[16], float
         codes[t][0] = codes[t][1] = 0;
         float e = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float s = v[i] * mul;
-            const uint32_t c = e2m1_rn(s);
-            const float d = (e2m1_value(c) - s) * sfd;      // error in units of x * ge
-            e += d * d;
+        for (int i = 0; i < 16; i += 2) {
+            const float s0 = v[i] * mul, s1 = v[i + 1] * mul;
+            const uint32_t c = e2m1x2_rn(s0, s1);
+            const float2 q = e2m1x2_value(c);
+            // error in units of x * ge; the operations are spelled out because nearly equal sums decide here
+            const float d0 = __fmul_rn(__fsub_rn(q.x, __fmul_rn(v[i], mul)), sfd), d1 = __fmul_rn(__fsub_rn(q.y, __fmul_rn(v[i + 1], mul)), sfd);
+            e = __fmaf_rn(d1, d1, __fmaf_rn(d0, d0, e));
             codes[t][i >> 3] |= c << ((i & 7) * 4);
         }
         err[t] = e;
@@ -139,9 +135,9 @@ __device__ __forceinline__ uint8_t quant_block16_4o6(const float (&v)[16], float
         err[1] += __shfl_xor_sync(0xffffffffu, err[1], o);
     }
     const int pick = err[1] < err[0] ? 1 : 0;
-    out[0] = codes[pick][0];
-    out[1] = codes[pick][1];
-    return sfb[pick];
+    out[0] = pick ? codes[1][0] : codes[0][0];
+    out[1] = pick ? codes[1][1] : codes[0][1];
+    return pick ? sfb[1] : sfb[0];
 }
 
 __device__ __forceinline__ void load16(const bf16* p, float (&v)[16]) {
@@ -175,35 +171,65 @@ __device__ __forceinline__ void hadamard16(float (&v)[16], uint32_t sign_mask) {
     for (int i = 0; i < 16; ++i) v[i] *= 0.25f;
 }
 
+// ------------------------------------------------------------------------------------------ output tile
+// Both quantisers work on tiles of 128 output rows x 128 elements (8 blocks of 16): the codes (64 bytes a row) and the scales (two
+// 512-byte atoms) are collected in shared memory and leave as whole sectors.  Written straight from the threads that compute them, each
+// scale is a one-byte store into a sector of its own, and the codes of a transpose are 8-byte stores a whole row apart.
+constexpr int QT_ROWS = 128, QT_COLS = 128, QT_BLOCKS = QT_COLS / 16, QT_PITCH = QT_COLS / 2 + 8;
+struct QTile {
+    uint8_t q[QT_ROWS * QT_PITCH];
+    alignas(16) uint8_t sf[QT_ROWS * QT_BLOCKS];
+    __device__ __forceinline__ void put(int r, int b, const uint32_t (&codes)[2], uint8_t scale) {
+        *reinterpret_cast<uint2*>(q + r * QT_PITCH + b * 8) = make_uint2(codes[0], codes[1]);
+        sf[(b >> 2) * 512 + (r & 31) * 16 + (r >> 5) * 4 + (b & 3)] = scale;
+    }
+    // `rows` x `kblocks`: the whole output; (row0, kb0): this tile's origin.  Scales of rows and blocks behind the end are zero, so the
+    // buffer needs no clearing beforehand.
+    __device__ __forceinline__ void write(uint8_t* __restrict__ qg, uint8_t* __restrict__ sfg, int row0, int kb0, int rows, int kblocks, int atoms_k) const {
+        for (int i = threadIdx.x; i < QT_ROWS * QT_BLOCKS; i += blockDim.x) {
+            const int r = i / QT_BLOCKS, b = i % QT_BLOCKS;
+            if (row0 + r < rows && kb0 + b < kblocks)
+                *reinterpret_cast<uint2*>(qg + (static_cast<size_t>(row0 + r) * kblocks + kb0 + b) * 8) = *reinterpret_cast<const uint2*>(q + r * QT_PITCH + b * 8);
+        }
+        const int atom0 = kb0 >> 2;
+        if (threadIdx.x < 64 && atom0 + (threadIdx.x >> 5) < atoms_k)
+            reinterpret_cast<uint4*>(sfg + (static_cast<size_t>(row0 >> 7) * atoms_k + atom0) * 512)[threadIdx.x] = reinterpret_cast<const uint4*>(sf)[threadIdx.x];
+    }
+};
+
 // ------------------------------------------------------------------------------------------ row-wise quantise
 // x [rows, K] bf16 (K % 16 == 0) -> q [rows, K/2] bytes, sf in atom layout.  block2d: scales are shared by 16x16 tiles (rows % 16 == 0).
+// 256 threads per 128 x 128 tile, four blocks each.  Bound by instruction issue: about 12 per element with four-over-six (both
+// candidates' codes and error sums), about 30 with stochastic rounding (the hash).  24576 x 4096 on B200: four-over-six 958 -> 95 us
+// (2.7 TB/s of the 258 MB it must move), plain 151 -> 64 us, stochastic 476 -> 197 us; before, the codes came from a chain of compares,
+// their values from a table in local memory, and every scale byte was a store of its own.
 template <bool SR>
 __global__ void __launch_bounds__(256) nvfp4_quantize_rows_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                                   const float* __restrict__ amax_tensor, int rows, int K, int atoms_k, uint32_t seed,
                                                                   int block2d, int four_over_six) {
+    __shared__ QTile out_tile;
     const float at = __ldg(amax_tensor);
     const float ge = at > 0.f ? __fdiv_rn(four_over_six ? 1536.f : 2688.f, at) : 1.f;
     const int kblocks = K / 16;
-    const size_t total = static_cast<size_t>(rows) * kblocks;
-    // warp-uniform trip count: the 16x16-tile path shuffles across lanes
-    for (size_t base = blockIdx.x * static_cast<size_t>(blockDim.x) + (threadIdx.x & ~31); base < total; base += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t b = base + (threadIdx.x & 31);
-        const bool live = b < total;   // total is a multiple of 16 in the tile path, so 16-lane groups are all-live or all-dead
-        int r = 0, kb = 0;
-        if (!live) {
-        } else if (block2d) {   // consecutive threads walk down the 16 rows of a tile so the tile abs-max is a 16-lane shuffle
-            const size_t tile = b >> 4;
-            const int tiles_k = kblocks;
-            r = static_cast<int>(tile / tiles_k) * 16 + static_cast<int>(b & 15);
-            kb = static_cast<int>(tile % tiles_k);
+    const int tiles_k = (kblocks + QT_BLOCKS - 1) / QT_BLOCKS;
+    const int row0 = static_cast<int>(blockIdx.x / tiles_k) * QT_ROWS, kb0 = static_cast<int>(blockIdx.x % tiles_k) * QT_BLOCKS;
+#pragma unroll 1
+    for (int it = 0; it < QT_ROWS * QT_BLOCKS / 256; ++it) {
+        int r, b;
+        if (block2d) {   // lanes walk down the 16 rows of a 16x16 tile, so that its abs-max and its decision are 16-lane shuffles
+            const int tile = it * 16 + (threadIdx.x >> 4);
+            r = (tile / QT_BLOCKS) * 16 + (threadIdx.x & 15);
+            b = tile % QT_BLOCKS;
         } else {
-            r = static_cast<int>(b / kblocks);
-            kb = static_cast<int>(b % kblocks);
+            const int i = it * 256 + threadIdx.x;
+            r = i / QT_BLOCKS;
+            b = i % QT_BLOCKS;
         }
+        const bool live = row0 + r < rows && kb0 + b < kblocks;   // rows is a multiple of 16 in the tile path: 16-lane groups agree
         float v[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = 0.f;
-        if (live) load16(x + static_cast<size_t>(r) * K + kb * 16, v);
+        if (live) load16(x + static_cast<size_t>(row0 + r) * K + (kb0 + b) * 16, v);
         float forced = -1.f;
         if (block2d) {
             float m = 0.f;
@@ -215,53 +241,60 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_rows_kernel(const bf16* __
         }
         uint32_t out[2];
         uint8_t sfb;
-        if (!SR && four_over_six) {
-            sfb = quant_block16_4o6(v, ge, forced, out, block2d ? 16 : 1);   // before the `live` test: the tile decision is a lane shuffle
-            if (!live) continue;
-        } else {
-            if (!live) continue;
-            sfb = quant_block16<SR>(v, ge, forced, seed, static_cast<uint64_t>(r) * K + kb * 16, out);
-        }
-        *reinterpret_cast<uint2*>(q + static_cast<size_t>(r) * (K / 2) + kb * 8) = make_uint2(out[0], out[1]);
-        sf[sf_offset(r, kb, atoms_k)] = sfb;
+        if (!SR && four_over_six) sfb = quant_block16_4o6(v, ge, forced, out, block2d ? 16 : 1);
+        else sfb = quant_block16<SR>(v, ge, forced, seed, static_cast<uint64_t>(row0 + r) * K + (kb0 + b) * 16, out);
+        out_tile.put(r, b, out, live ? sfb : static_cast<uint8_t>(0));
     }
+    __syncthreads();
+    out_tile.write(q, sf, row0, kb0, rows, kblocks, atoms_k);
 }
 
 // ------------------------------------------------------------------------------------------ transpose-quantise
 // x [R, C] bf16 -> quantised x^T: q [C, R/2], sf for (row = c, block = r/16).  R % 64 == 0, C % 64 == 0.
+// The 128 x 128 input tile passes through shared memory as bf16; a lane owns two adjacent columns (4-byte reads, no bank conflicts).
+// 24576 x 4096 on B200: four-over-six 1284 -> 98 us, with the Hadamard transform 1316 -> 118 us, stochastic with it 349 -> 221 us.
+constexpr int QX_PITCH = QT_ROWS + 8;     // bf16 elements per staged row
 template <bool SR, bool RHT>
 __global__ void __launch_bounds__(256) nvfp4_quantize_transpose_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                                        const float* __restrict__ amax_tensor, int R, int C, int atoms_k, uint32_t seed,
                                                                        uint32_t sign_mask, int four_over_six) {
-    __shared__ float tile[64][65];
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x) {   // 64 rows x 8 vectors of 8
-        const int rr = i >> 3, cv = (i & 7) * 8;
-        const uint4 raw = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r0 + rr) * C + c0 + cv);
-        const bf162* p = reinterpret_cast<const bf162*>(&raw);
+    __shared__ QTile out_tile;
+    __shared__ alignas(16) bf16 tile[QT_COLS * QX_PITCH];
+    const int tiles_c = (C + QT_ROWS - 1) / QT_ROWS;
+    const int c0 = static_cast<int>(blockIdx.x % tiles_c) * QT_ROWS, r0 = static_cast<int>(blockIdx.x / tiles_c) * QT_COLS;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(p[j]);
-            tile[rr][cv + 2 * j] = f.x;
-            tile[rr][cv + 2 * j + 1] = f.y;
-        }
+    for (int it = 0; it < QT_COLS * QT_ROWS / 8 / 256; ++it) {
+        const int i = it * 256 + threadIdx.x, rr = i / (QT_ROWS / 8), cv = (i % (QT_ROWS / 8)) * 8;
+        uint4 raw = make_uint4(0, 0, 0, 0);
+        if (r0 + rr < R && c0 + cv < C) raw = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r0 + rr) * C + c0 + cv);
+        *reinterpret_cast<uint4*>(tile + rr * QX_PITCH + cv) = raw;
     }
     __syncthreads();
     const float at = __ldg(amax_tensor);
     // the Hadamard transform is orthonormal, so the tensor abs-max bound grows by at most 4x; keep head-room for it
     const float enc = (!SR && four_over_six) ? 1536.f : 2688.f;
     const float ge = at > 0.f ? (RHT ? enc / (at * 2.f) : enc / at) : 1.f;
-    const int c = threadIdx.x & 63, rb = threadIdx.x >> 6;   // column, 16-row block within the tile
-    float v[16];
+#pragma unroll 1
+    for (int it = 0; it < QT_ROWS / 2 * QT_BLOCKS / 256; ++it) {
+        const int i = it * 256 + threadIdx.x, pair = i % (QT_ROWS / 2), rb = i / (QT_ROWS / 2);   // columns 2 pair, 2 pair + 1; 16-row block
+        bf162 raw[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = tile[rb * 16 + i][c];
-    if (RHT) hadamard16(v, sign_mask);
-    uint32_t out[2];
-    const int kb = (r0 >> 4) + rb;
-    const uint8_t sfb = (!SR && four_over_six) ? quant_block16_4o6(v, ge, -1.f, out, 1)
-                                                : quant_block16<SR>(v, ge, -1.f, seed, static_cast<uint64_t>(c0 + c) * R + r0 + rb * 16, out);
-    *reinterpret_cast<uint2*>(q + static_cast<size_t>(c0 + c) * (R / 2) + (r0 + rb * 16) / 2) = make_uint2(out[0], out[1]);
-    sf[sf_offset(c0 + c, kb, atoms_k)] = sfb;
+        for (int k = 0; k < 16; ++k) raw[k] = *reinterpret_cast<const bf162*>(tile + (rb * 16 + k) * QX_PITCH + 2 * pair);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = 2 * pair + h;
+            float v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = __bfloat162float(h ? raw[k].y : raw[k].x);
+            if (RHT) hadamard16(v, sign_mask);
+            uint32_t out[2];
+            const uint8_t sfb = (!SR && four_over_six) ? quant_block16_4o6(v, ge, -1.f, out, 1)
+                                                        : quant_block16<SR>(v, ge, -1.f, seed, static_cast<uint64_t>(c0 + c) * R + r0 + rb * 16, out);
+            out_tile.put(c, rb, out, c0 + c < C && r0 + rb * 16 < R ? sfb : static_cast<uint8_t>(0));
+        }
+    }
+    __syncthreads();
+    out_tile.write(q, sf, c0, r0 >> 4, C, R >> 4, atoms_k);
 }
 
 // ------------------------------------------------------------------------------------------ dequantise
@@ -294,14 +327,17 @@ static int q_grid(size_t items, int num_sms) {
 void nvfp4_quantize_rows(const void* x, void* q, void* sf, const float* amax_tensor, int rows, int K, int stochastic, uint32_t seed, int block2d,
                          int num_sms, cudaStream_t s, int four_over_six) {
     const int atoms_k = (K / 16 + 3) / 4;
-    const int grid = q_grid(static_cast<size_t>(rows) * (K / 16), num_sms);
+    (void)num_sms;
+    if (rows <= 0 || K <= 0) return;
+    const unsigned grid = static_cast<unsigned>((rows + QT_ROWS - 1) / QT_ROWS) * static_cast<unsigned>((K / 16 + QT_BLOCKS - 1) / QT_BLOCKS);
     if (stochastic) nvfp4_quantize_rows_kernel<true><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, (uint8_t*)sf, amax_tensor, rows, K, atoms_k, seed, block2d, 0);
     else nvfp4_quantize_rows_kernel<false><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, (uint8_t*)sf, amax_tensor, rows, K, atoms_k, seed, block2d, four_over_six);
 }
 void nvfp4_quantize_transpose(const void* x, void* q, void* sf, const float* amax_tensor, int R, int C, int stochastic, int hadamard, uint32_t seed,
                               uint32_t sign_mask, cudaStream_t s, int four_over_six) {
     const int atoms_k = (R / 16 + 3) / 4;
-    const dim3 grid(C / 64, R / 64);
+    if (R <= 0 || C <= 0) return;
+    const unsigned grid = static_cast<unsigned>((C + QT_ROWS - 1) / QT_ROWS) * static_cast<unsigned>((R + QT_COLS - 1) / QT_COLS);
     const bf16* xp = (const bf16*)x;
     uint8_t* qp = (uint8_t*)q;
     uint8_t* sp = (uint8_t*)sf;

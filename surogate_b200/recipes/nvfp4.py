@@ -21,7 +21,7 @@ Parity: csrc/src/recipes/nvfp4/nvfp4_recipe.cpp:629-1131, recipes/nvfp4/kernels/
 """
 from __future__ import annotations
 
-from typing import Dict, Tuple
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -35,10 +35,10 @@ HADAMARD_SIGNS = 0b1011001110001101
 
 
 class Fp4Tensor:
-    __slots__ = ("q", "sf", "inv_ge")
+    __slots__ = ("q", "sf", "inv_ge", "amax")
 
-    def __init__(self, q, sf, inv_ge):
-        self.q, self.sf, self.inv_ge = q, sf, inv_ge
+    def __init__(self, q, sf, inv_ge, amax):
+        self.q, self.sf, self.inv_ge, self.amax = q, sf, inv_ge, amax
 
 
 class NVFP4Recipe(GroupedFp8Mixin, Recipe):
@@ -82,25 +82,28 @@ class NVFP4Recipe(GroupedFp8Mixin, Recipe):
         self.calls += 1
         return (self.step * 7919 + self.calls * 104729) & 0x7FFFFFFF
 
-    def _q_rows(self, x: torch.Tensor, sr: bool = False, block2d: bool = False) -> Fp4Tensor:
+    def _q_rows(self, x: torch.Tensor, sr: bool = False, block2d: bool = False, am: Optional[torch.Tensor] = None) -> Fp4Tensor:
         x = x.contiguous()
-        am = self._amax(x)
+        am = self._amax(x) if am is None else am
         fos = self.four_over_six and not sr
         q, sf = self.ext.nvfp4_quantize(x, am, sr, self._seed() if sr else 0, block2d, fos)
-        return Fp4Tensor(q, sf, am / (ENCODE_4O6 if fos else ENCODE))
+        return Fp4Tensor(q, sf, am / (ENCODE_4O6 if fos else ENCODE), am)
 
-    def _q_transpose(self, x: torch.Tensor, sr: bool, rht: bool) -> Fp4Tensor:
+    def _q_transpose(self, x: torch.Tensor, sr: bool, rht: bool, am: Optional[torch.Tensor] = None) -> Fp4Tensor:
         x = x.contiguous()
-        am = self._amax(x)
+        am = self._amax(x) if am is None else am
         fos = self.four_over_six and not sr
         q, sf = self.ext.nvfp4_quantize_transpose(x, am, sr, rht, self._seed() if sr else 0, HADAMARD_SIGNS, fos)
-        return Fp4Tensor(q, sf, am * (2.0 if rht else 1.0) / (ENCODE_4O6 if fos else ENCODE))
+        return Fp4Tensor(q, sf, am * (2.0 if rht else 1.0) / (ENCODE_4O6 if fos else ENCODE), am)
 
     def _weight(self, ctx, role: str, w: torch.Tensor, transposed: bool) -> Fp4Tensor:
         key = (ctx.layer, role, transposed)
         t = self.weight_cache.get(key)
         if t is None:
-            t = self._q_transpose(w, False, False) if transposed else self._q_rows(w, False, block2d=True)
+            # both orientations of a weight share one abs-max pass
+            other = self.weight_cache.get((ctx.layer, role, not transposed))
+            am = other.amax if other is not None else None
+            t = self._q_transpose(w, False, False, am) if transposed else self._q_rows(w, False, block2d=True, am=am)
             self.weight_cache[key] = t
         return t
 
@@ -137,7 +140,7 @@ class NVFP4Recipe(GroupedFp8Mixin, Recipe):
         dx = self._gemm(dyq, self._weight(ctx, role, w, True))              # [M, N] . (W^T [K, N])^T
         tgt, acc = ctx.grad_target(op.outputs[1])
         if tgt is not None:
-            a = self._q_transpose(dy2, self.stochastic, self.hadamard)       # dy^T [N, M]
+            a = self._q_transpose(dy2, self.stochastic, self.hadamard, dyq.amax)   # dy^T [N, M]
             b = self._q_transpose(x2, False, self.hadamard)                  # x^T  [K, M]
             self._gemm(a, b, tgt, accumulate=acc)
         return dx, None

@@ -149,3 +149,49 @@ def test_gemm_with_four_over_six_operands(ext):
     da, db = ext.nvfp4_dequantize(qa, sfa, am_a, 1.0, 1536.0), ext.nvfp4_dequantize(qb, sfb, am_b, 1.0, 1536.0)
     assert _rel(d, da.float() @ db.float().t()) < 6e-3
     assert _rel(d, a.float() @ b.float().t()) < 0.2
+
+
+def _sr_codes(s, seed, idx):
+    """Stochastic rounding as the kernels define it: splitmix64 of the element index gives u in [0, 1); the upper grid neighbour is
+    taken when u is below the position between the neighbours."""
+    import numpy as np
+
+    z = idx.astype(np.uint64) + np.uint64((0x9E3779B97F4A7C15 * (seed + 1)) % 2 ** 64)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    z ^= z >> np.uint64(31)
+    u = (z >> np.uint64(40)).astype(np.float64) / 2.0 ** 24
+    grid = np.array([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
+    a = np.minimum(np.abs(s.astype(np.float64)), 6.0)
+    lo = np.searchsorted(grid, a, side="right") - 1
+    nxt = np.minimum(lo + 1, 7)
+    p = (a - grid[lo]) / np.maximum(grid[nxt] - grid[lo], 0.5)
+    return np.where(u < p, nxt, lo) + 8 * (s < 0)
+
+
+@pytest.mark.parametrize("transpose,rows,K", [(False, 16, 16), (False, 129, 48), (False, 200, 400), (False, 384, 272),
+                                              (True, 64, 64), (True, 192, 320), (True, 320, 192)])
+@pytest.mark.parametrize("stochastic", [False, True])
+def test_quantisers_at_the_edges_of_their_tiles(ext, transpose, rows, K, stochastic):
+    """Sizes below, between and just above the 128 x 128 tiles (`rows` x `K` is the quantised shape): codes against the emulation, and
+    zero scales in the padding rows and blocks, which the tensor core reads."""
+    import numpy as np
+    from surogate_b200.ops import nvfp4_ref as ref
+
+    torch.manual_seed(rows + K)
+    x = (torch.randn(rows, K, device=DEV) * torch.rand(rows, 1, device=DEV) * 3).bfloat16()
+    x[0, 0] = -0.0
+    amax = x.float().abs().max().reshape(1)
+    q, sf = ext.nvfp4_quantize_transpose(x.t().contiguous(), amax, stochastic, False, 11, 0) if transpose else ext.nvfp4_quantize(x, amax, stochastic, 11, False)
+    codes, sfd, ge = ref.quantize(x.float(), amax[0])
+    sf_all = ref.atoms_to_sf(sf, (rows + 127) // 128 * 128, (K // 16 + 3) // 4 * 4)
+    sf_got = sf_all[:rows, :K // 16].view(torch.float8_e4m3fn).float()
+    assert not sf_all[rows:].any() and not sf_all[:, K // 16:].any()
+    sf_bad = sf_got != sfd
+    assert sf_bad.float().mean().item() < 5e-3
+    if stochastic:
+        s = (x.float().view(rows, -1, 16) * torch.where(sfd > 0, ge / sfd, torch.zeros_like(sfd)).unsqueeze(-1)).view(rows, K).cpu().numpy()
+        idx = np.arange(rows * K, dtype=np.uint64).reshape(rows, K)
+        codes = torch.from_numpy(_sr_codes(s, 11, idx).astype(np.int64)).to(DEV)
+    wrong = (ref.unpack_codes(q) != codes) & (~sf_bad).repeat_interleave(16, dim=1)
+    assert wrong.float().mean().item() < 2e-3       # a product on a rounding boundary may fall the other way
