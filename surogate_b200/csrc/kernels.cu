@@ -206,13 +206,37 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const bf16* __r
         }
     }
 }
-// out[c] += sum over a slice of the partial rows (gridDim.y slices; ``out`` is zeroed by the launcher)
-__global__ void column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int nblocks, int C) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    float s = 0.f;
-    for (int b = blockIdx.y; b < nblocks; b += gridDim.y) s += partial[static_cast<size_t>(b) * C + c];
-    atomicAdd(out + c, s);
+// out[c] = sum of the partial rows.  One CTA per 16 columns: four lanes x 16 bytes span the columns, 256 rows are read side by side, so
+// that a thread has its few loads in flight together, and the sums meet by shuffle and in shared memory (fixed order, no atomics, no
+// cleared output).  Latency-bound: a few us, where 32 CTAs whose threads walked 148 rows each, with an
+// atomic per slice and a memset before it, took 43 us for [1184, 1024].  RMSNorm backward of 16384 x 1024 on B200 83 -> 51 us in all,
+// 1024 x 512 43 -> 13 us, 8192 x 4096 90 -> 74 us.
+constexpr int CS_COLS = 16, CS_THREADS = 1024;
+__global__ void __launch_bounds__(CS_THREADS) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int nblocks, int C) {
+    __shared__ float sh[CS_THREADS / 32][CS_COLS];
+    const int c = blockIdx.x * CS_COLS + (threadIdx.x & 3) * 4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < C) {
+#pragma unroll 4
+        for (int b = threadIdx.x >> 2; b < nblocks; b += CS_THREADS / 4) {
+            const float4 v = *reinterpret_cast<const float4*>(partial + static_cast<size_t>(b) * C + c);
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+    }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane < 4) *reinterpret_cast<float4*>(&sh[warp][lane * 4]) = s;
+    __syncthreads();
+    if (threadIdx.x < CS_COLS && blockIdx.x * CS_COLS + threadIdx.x < C) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < CS_THREADS / 32; ++w) t += sh[w][threadIdx.x];
+        out[blockIdx.x * CS_COLS + threadIdx.x] = t;
+    }
 }
 
 // ------------------------------------------------------------------------------------------ SwiGLU
@@ -939,9 +963,7 @@ void rmsnorm_bwd_n(const void* dy, const void* x, const void* w, const float* rs
         default: SG_RB(8); break;
     }
 #undef SG_RB
-    cudaMemsetAsync(dw, 0, static_cast<size_t>(C) * sizeof(float), s);
-    const int slices = blocks >= 64 ? 8 : 1;
-    column_sum_kernel<<<dim3((C + 255) / 256, slices), 256, 0, s>>>(dw_partial, dw, blocks, C);
+    column_sum_kernel<<<(C + CS_COLS - 1) / CS_COLS, CS_THREADS, 0, s>>>(dw_partial, dw, blocks, C);
 }
 void rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* d_res, void* dx, float* dw_partial, float* dw, int rows,
                  int C, int num_sms, cudaStream_t s) {

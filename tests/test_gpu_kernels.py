@@ -174,6 +174,19 @@ def test_rmsnorm_fwd_bwd(ext, C):
     assert abs(amax.item() - yref.abs().max().item()) < 0.02 * amax.item()
 
 
+@pytest.mark.parametrize("rows,C", [(5, 24), (300, 1000), (3000, 1024), (257, 4104), (40, 16384)])
+def test_rmsnorm_weight_gradient_sums(ext, rows, C):
+    """The column sums behind dw: widths that are no multiple of a CTA's 16 columns, fewer partial rows than a CTA reads side by side, and
+    many.  fp32 sums of `rows` products against fp64: a few 2^-24 of the largest column sum of magnitudes."""
+    torch.manual_seed(rows + C)
+    dy, x, w = (torch.randn(*s, device=DEV).bfloat16() for s in ((rows, C), (rows, C), (C,)))
+    rstd = torch.rand(rows, device=DEV) + 0.5
+    _, dw = ext.rmsnorm_bwd(dy, x, w, rstd, None)
+    terms = dy.double() * x.double() * rstd.double()[:, None]
+    assert ((dw.double() - terms.sum(0)).abs() <= 16 * 2.0 ** -24 * terms.abs().sum(0)).all()
+    assert torch.equal(dw, ext.rmsnorm_bwd(dy, x, w, rstd, None)[1])
+
+
 def test_swiglu(ext):
     rows, M = 517, 3072
     x = torch.randn(rows, 2 * M, device=DEV).bfloat16()
