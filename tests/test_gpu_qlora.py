@@ -44,3 +44,29 @@ def test_qlora_step_runs_on_the_cuda_dequantisers():
     losses = [tr.step(tok[:, :-1], tok[:, 1:])["loss"] for _ in range(6)]
     assert losses[-1] < losses[0] - 0.05, losses
     assert ext().launch_count() > before
+
+
+@pytest.mark.parametrize("n,block", [(8, 8), (264, 24), (9896, 64), (1 << 18, 256), (1237 * 320, 320)])
+@pytest.mark.parametrize("double_quant", [False, True])
+def test_nf4_dequantiser_sizes_and_block_lengths(n, block, double_quant):
+    """Counts below one warp, with a ragged tail, and blocks that are and are not a power of two (the block index is a shift or a division):
+    the product of level and abs-max in fp32, rounded once, so the bits are the emulation's."""
+    from surogate_b200.ops import ext
+    from surogate_b200.quant import codecs
+
+    e = ext()
+    g = torch.Generator(device="cuda").manual_seed(n + block)
+    codes = torch.randint(0, 256, ((n // 2 + 7) // 8 * 8,), generator=g, device="cuda", dtype=torch.uint8)
+    nb = (n + block - 1) // block
+    absmax = torch.rand(nb, generator=g, device="cuda") + 0.1
+    args = (absmax, None, None)
+    if double_quant:
+        q = torch.randint(-128, 128, (nb,), generator=g, device="cuda", dtype=torch.int8)
+        scale, offset = torch.full(((nb + 255) // 256,), 2.0 ** -8, device="cuda"), torch.full((1,), 0.75, device="cuda")   # exact in fp32
+        absmax = q.float() * 2.0 ** -8 + 0.75
+        args = (q, scale, offset)
+    out = e.dequant_blockwise("bnb_nf4", codes, *args, n, block)
+    levels = torch.as_tensor(codecs.NF4_LEVELS, dtype=torch.float32, device="cuda")
+    idx = torch.stack([codes & 15, codes >> 4], -1).reshape(-1)[:n].long()
+    want = (levels[idx] * absmax.repeat_interleave(block)[:n]).bfloat16()
+    assert torch.equal(out, want)
