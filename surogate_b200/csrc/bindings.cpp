@@ -93,6 +93,14 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& d, bool a_mn, bool b_mn, boo
     if (const char* v = std::getenv("SUROGATE_GEMM_GROUP_M")) p.pair_group_m = std::atoi(v);
     sg::GemmOperand A{a.data_ptr(), static_cast<uint64_t>(a.stride(0)) * es};
     sg::GemmOperand B{b.data_ptr(), static_cast<uint64_t>(b.stride(0)) * es};
+    // pieces of a split contraction and their counters: from the caching allocator, on the stream that uses them
+    const sg::GemmPlan plan = sg::gemm_plan_sm100(p, num_sms());
+    Tensor ws;
+    if (plan.splits > 1) {
+        ws = torch::empty({static_cast<int64_t>(plan.workspace_floats + plan.num_counters)}, d.options().dtype(at::kFloat));
+        p.workspace = ws.data_ptr<float>();
+        p.counters = reinterpret_cast<int*>(p.workspace + plan.workspace_floats);
+    }
     g_launches += 1;
     const char* err = sg::gemm_sm100(A, B, p, num_sms(), cur_stream());
     TORCH_CHECK(err == nullptr, err ? err : "");

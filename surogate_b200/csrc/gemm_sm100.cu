@@ -163,6 +163,73 @@ __device__ __forceinline__ void store_direct_32(const GemmParams& p, const TileI
 
 constexpr int MAX_GROUPS = 256;
 
+// ------------------------------------------------------------------------------------------------ units of work
+// A unit is one output tile, or one of `splits` equal pieces of its contraction.  Whole waves of tiles stay whole; only the tiles from
+// `split_from` on are cut, so that the last wave (or the only one, for small outputs with a long contraction) fills the chip.  A piece
+// leaves its fp32 accumulator in the workspace; the warp that arrives last at its 32 rows adds the pieces in order of the contraction
+// (the same order in every run) and stores the result.  Nobody waits for anybody.
+struct Unit {
+    int tile, kb0, kb1;
+    int piece;   // -1: a whole tile
+};
+__device__ __forceinline__ int num_units(const GemmParams& p, int num_tiles) {
+    return p.splits > 1 ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
+}
+__device__ __forceinline__ Unit get_unit(const GemmParams& p, int num_tiles, int num_k, int unit) {
+    if (p.splits <= 1 || unit < p.split_from) return Unit{unit, 0, num_k, -1};
+    const int r = unit - p.split_from, n = num_tiles - p.split_from;
+    const int s = r / n;
+    return Unit{p.split_from + r % n, s * num_k / p.splits, (s + 1) * num_k / p.splits, s};
+}
+// Workspace of one warp's 32 rows x COLS columns: 16-byte vectors, lanes side by side (whole lines per store), pieces `stride` floats apart.
+// `valid` = columns that exist.
+template <int COLS> __device__ __forceinline__ void park_piece(uint32_t t_row, float4* ws, int lane, int valid) {
+#pragma unroll 1
+    for (int c = 0; c < COLS && c < valid; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(t_row + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            ws[(c / 4 + j) * 32 + lane] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+    }
+}
+__device__ __forceinline__ void sum_pieces(const float4* ws, size_t stride, int pieces, int lane, int c, uint32_t (&r)[32]) {
+    float4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __ldcg(ws + (c / 4 + j) * 32 + lane);
+    // the next piece is requested before this one is added
+    float4 w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = __ldcg(ws + stride + (c / 4 + j) * 32 + lane);
+    for (int s = 1; s < pieces; ++s) {
+        float4 x[8];
+        const size_t next = (s + 1 < pieces ? s + 1 : s) * stride;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = __ldcg(ws + next + (c / 4 + j) * 32 + lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { v[j].x += w[j].x; v[j].y += w[j].y; v[j].z += w[j].z; v[j].w += w[j].w; w[j] = x[j]; }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        r[4 * j] = __float_as_uint(v[j].x);
+        r[4 * j + 1] = __float_as_uint(v[j].y);
+        r[4 * j + 2] = __float_as_uint(v[j].z);
+        r[4 * j + 3] = __float_as_uint(v[j].w);
+    }
+}
+// True in the warp that completes these rows: all pieces are in the workspace and visible to it.
+__device__ __forceinline__ bool last_piece(int* counter, int pieces, int lane) {
+    __threadfence();
+    __syncwarp();
+    int old = 0;
+    if (lane == 0) old = atomicAdd(counter, 1);
+    old = __shfl_sync(0xffffffffu, old, 0);
+    if (old != pieces - 1) return false;
+    __threadfence();
+    return true;
+}
+
 template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
@@ -223,6 +290,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
     const int num_tiles = num_tiles_sh;
+    const int units = num_units(p, num_tiles);      // grouped problems are never split: a unit is a tile
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -233,10 +301,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int b_chunks = p.b_mn ? (BN * p.elem_bytes) / TILE_K_BYTES : 1;
             const int chunk_bytes = BK * TILE_K_BYTES;   // MN-major chunk: BK rows of 128 B
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const TileInfo t = get_tile<BN>(p, tile_start, tile, BK);
+            for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+                const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
+                const TileInfo t = get_tile<BN>(p, tile_start, u.tile, BK);
                 const int m0 = t.a_row0, n0 = t.b_row0;
-                for (int kb = 0; kb < t.num_k; ++kb) {
+                const int kb1 = u.piece < 0 ? t.num_k : u.kb1;
+                for (int kb = u.kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, &abort_flag)) { ok = false; break; }
                     const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
                     const uint32_t sb = sa + A_STAGE_BYTES;
@@ -268,13 +338,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const uint32_t a_kstep = p.a_mn ? (BK / 4) * TILE_K_BYTES : 32;
             const uint32_t b_kstep = p.b_mn ? (BK / 4) * TILE_K_BYTES : 32;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+            for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local_tile) {
                 const int acc = local_tile & 1;
                 if (!mbar_wait(tempty_bar(acc), acc_phase[acc] ^ 1u, &abort_flag)) { ok = false; break; }
                 acc_phase[acc] ^= 1u;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                const int num_k = get_tile<BN>(p, tile_start, tile, BK).num_k;
+                const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
+                const int num_k = u.piece < 0 ? get_tile<BN>(p, tile_start, u.tile, BK).num_k : u.kb1 - u.kb0;
                 for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, &abort_flag)) { ok = false; break; }
                     tc_fence_after();
@@ -304,14 +375,33 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (p.scale_b) scale *= __ldg(p.scale_b);
         float amax = 0.f;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
-            const TileInfo t = get_tile<BN>(p, tile_start, tile, BK);
+        for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local_tile) {
+            const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
+            const TileInfo t = get_tile<BN>(p, tile_start, u.tile, BK);
             const int acc = local_tile & 1;
             if (!mbar_wait(tfull_bar(acc), acc_phase[acc], &abort_flag)) { ok = false; break; }
             acc_phase[acc] ^= 1u;
             tc_fence_after();
             const int row = t.d_row0 + quad * 32 + lane;
             const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
+            if (u.piece >= 0) {
+                const int slot = (u.tile - p.split_from) * 4 + quad, slots = (num_tiles - p.split_from) * 4;
+                float4* ws = reinterpret_cast<float4*>(p.workspace) + static_cast<size_t>(slot) * (32 * BN / 4);
+                const size_t stride = static_cast<size_t>(slots) * (32 * BN / 4);
+                const bool rows = t.d_row0 + quad * 32 < t.m_end;        // the same in every piece of the tile
+                if (rows) park_piece<BN>(t_row, ws + u.piece * stride, lane, t.n_end - t.d_col0);
+                tc_fence_before();
+                mbar_arrive(tempty_bar(acc));
+                if (rows && last_piece(p.counters + slot, p.splits, lane)) {
+#pragma unroll 1
+                    for (int c = 0; c < BN && t.d_col0 + c < t.n_end; c += 32) {
+                        uint32_t r[32];
+                        sum_pieces(ws, stride, p.splits, lane, c, r);
+                        store_direct_32(p, t, row, t.d_col0 + c, r, scale, amax);
+                    }
+                }
+                continue;
+            }
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 uint32_t r[32];
@@ -345,15 +435,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // fill 128 TMEM lanes x 256 columns in both CTAs.  Loads are per-CTA TMA copies (no cluster broadcast) that complete on the
 // leader's barrier; the MMA completion is committed to both CTAs' barriers.  The epilogue leaves through shared memory: every
 // warp packs its 32 rows x 128 bytes into a swizzled staging tile and one lane issues a TMA store (or a TMA add for fp32
-// accumulation), so global writes are whole 128-byte lines and the tensor map clips the edges.  bf16 accumulation and the
-// running abs-max of accumulated outputs keep the register path.  Dense problems only (mode 0).
+// accumulation), so global writes are whole 128-byte lines and the tensor map clips the edges.  bf16 accumulation (ACC) fetches D the
+// same way: a warp's four 32 x 64 tiles of D are requested into its staging tiles before the accumulator is complete, summed there in
+// fp32, rounded once and stored (8192 x 17408 += 16 deep on B200 643 -> 203 us, 151936 x 4096 += 4096 deep in FP8 2733 -> 1970 us; read
+// and added row by row from registers before).  Only an fp32 abs-max of accumulated values keeps the register
+// path.  Dense problems only (mode 0).
 constexpr int PAIR_BM = 256, PAIR_BN = 256;
 constexpr int PAIR_B_BYTES = 128 * TILE_K_BYTES;                 // this CTA's half of the B tile
 constexpr int PAIR_STAGE_BYTES = A_STAGE_BYTES + PAIR_B_BYTES;   // 32 KB
-constexpr int PAIR_STAGES = 6;
-constexpr int PAIR_EPI_WARP_BYTES = 2 * 4096;                    // two 32-row x 128-byte staging tiles per epilogue warp
-constexpr int PAIR_EPI_BYTES = 4 * PAIR_EPI_WARP_BYTES;
-constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_EPI_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+// staging tiles of 32 rows x 128 bytes per epilogue warp: two in turn, or with ACC one per 64-column chunk of D, paid for with one ring
+// stage (the ring is no slower with five: it is bound by operand bandwidth, not by latency)
+template <bool ACC> struct PairCfg {
+    static constexpr int STAGES = ACC ? 5 : 6;
+    static constexpr int EPI_BUFS = ACC ? 4 : 2;
+    static constexpr int EPI_WARP_BYTES = EPI_BUFS * 4096;
+    static constexpr int SMEM_BYTES = STAGES * PAIR_STAGE_BYTES + 4 * EPI_WARP_BYTES + 1024 /*align slack*/ + 384 /*barriers*/;
+};
 
 struct PairTile {
     int m0, n0;   // origin of the 256 x 256 tile
@@ -368,18 +465,22 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int tile) {
     return PairTile{(first_m + r % gsize) * PAIR_BM, (r / gsize) * PAIR_BN};
 }
 
+template <bool ACC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmD,
                  const GemmParams p, const int use_tma_store) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // same offset in both CTAs: the MMA applies one descriptor to both
+    constexpr int PAIR_STAGES = PairCfg<ACC>::STAGES;
     const uint32_t epi_base = smem_base + PAIR_STAGES * PAIR_STAGE_BYTES;
-    const uint32_t bar_base = epi_base + PAIR_EPI_BYTES;
-    // barriers (8 B each): full[STAGES] (used in the leader), empty[STAGES], tmem_full[2], tmem_empty[2] (used in the leader)
+    const uint32_t bar_base = epi_base + 4 * PairCfg<ACC>::EPI_WARP_BYTES;
+    // barriers (8 B each): full[STAGES] (used in the leader), empty[STAGES], tmem_full[2], tmem_empty[2] (used in the leader), with ACC
+    // d_full[4 warps][4 tiles]
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (PAIR_STAGES + s); };
     auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * PAIR_STAGES + a); };
     auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * PAIR_STAGES + 2 + a); };
+    auto d_bar = [&](int w, int b) { return bar_base + 8u * (2 * PAIR_STAGES + 4 + w * 4 + b); };
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
 
@@ -389,7 +490,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int BK = TILE_K_BYTES / p.elem_bytes;
     const int num_tiles = ((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
     const int num_k = (p.K + BK - 1) / BK;
-    const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+    const int units = num_units(p, num_tiles);
+    const int first_unit = blockIdx.x >> 1, unit_step = gridDim.x >> 1;
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -401,6 +503,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             mbar_init(tfull_bar(a), 1);
             mbar_init(tempty_bar(a), 8);      // one lane of each epilogue warp of both CTAs
         }
+        if (ACC)
+            for (int i = 0; i < 16; ++i) mbar_init(d_bar(i >> 2, i & 3), 1);
         fence_barrier_init();
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
@@ -425,33 +529,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int chunk_bytes = BK * TILE_K_BYTES;
             bool ok = true;
             // optional L2 prefetch cursor: runs `pair_prefetch` contraction blocks ahead of the load cursor (across tile boundaries)
-            int pf_tile = first_tile, pf_kb = 0, pf_m0 = 0, pf_n0 = 0;
+            int pf_unit = first_unit, pf_kb = 0, pf_end = 0, pf_m0 = 0, pf_n0 = 0;
             auto pf_origin = [&]() {
-                const PairTile t = pair_tile(p, pf_tile);
+                const Unit u = get_unit(p, num_tiles, num_k, pf_unit);
+                const PairTile t = pair_tile(p, u.tile);
+                pf_kb = u.kb0;
+                pf_end = u.kb1;
                 pf_m0 = t.m0 + static_cast<int>(rank) * 128;
                 pf_n0 = t.n0 + static_cast<int>(rank) * 128;
             };
             auto pf_step = [&]() {
-                if (pf_tile >= num_tiles) return;
+                if (pf_unit >= units) return;
                 const int k0 = pf_kb * BK;
                 if (!p.a_mn) tma_prefetch_l2_2d(&tmA, k0, pf_m0);
                 else for (int c = 0; c < a_chunks; ++c) tma_prefetch_l2_2d(&tmA, pf_m0 + c * BK, k0);
                 if (!p.b_mn) tma_prefetch_l2_2d(&tmB, k0, pf_n0);
                 else for (int c = 0; c < b_chunks; ++c) tma_prefetch_l2_2d(&tmB, pf_n0 + c * BK, k0);
-                if (++pf_kb == num_k) {
-                    pf_kb = 0;
-                    pf_tile += tile_step;
-                    if (pf_tile < num_tiles) pf_origin();
+                if (++pf_kb == pf_end) {
+                    pf_unit += unit_step;
+                    if (pf_unit < units) pf_origin();
                 }
             };
-            if (p.pair_prefetch > 0 && first_tile < num_tiles) {
+            if (p.pair_prefetch > 0 && first_unit < units) {
                 pf_origin();
                 for (int i = 0; i < PAIR_STAGES + p.pair_prefetch; ++i) pf_step();
             }
-            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
-                const PairTile t = pair_tile(p, tile);
+            for (int unit = first_unit; unit < units && ok; unit += unit_step) {
+                const Unit u = get_unit(p, num_tiles, num_k, unit);
+                const PairTile t = pair_tile(p, u.tile);
                 const int m0 = t.m0 + static_cast<int>(rank) * 128, n0 = t.n0 + static_cast<int>(rank) * 128;
-                for (int kb = 0; kb < num_k; ++kb) {
+                for (int kb = u.kb0; kb < u.kb1; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, &abort_flag)) { ok = false; break; }
                     if (p.pair_prefetch > 0) pf_step();
                     const uint32_t sa = smem_base + stage * PAIR_STAGE_BYTES;
@@ -485,13 +592,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const uint32_t a_kstep = p.a_mn ? (BK / 4) * TILE_K_BYTES : 32;
             const uint32_t b_kstep = p.b_mn ? (BK / 4) * TILE_K_BYTES : 32;
             bool ok = true;
-            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
+            for (int unit = first_unit; unit < units && ok; unit += unit_step, ++local_tile) {
                 const int acc = local_tile & 1;
                 if (!mbar_wait_cluster(tempty_bar(acc), acc_phase[acc] ^ 1u, &abort_flag)) { ok = false; break; }
                 acc_phase[acc] ^= 1u;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
-                for (int kb = 0; kb < num_k; ++kb) {
+                const Unit u = get_unit(p, num_tiles, num_k, unit);
+                for (int kb = 0; kb < u.kb1 - u.kb0; ++kb) {
                     if (!mbar_wait_cluster(full_bar(stage), phase, &abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + stage * PAIR_STAGE_BYTES;
@@ -521,32 +629,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         float amax = 0.f;
         bool ok = true;
         const uint32_t tempty_leader[2] = {mapa_shared(tempty_bar(0), 0), mapa_shared(tempty_bar(1), 0)};
-        const uint32_t stage_smem = epi_base + quad * PAIR_EPI_WARP_BYTES;
+        const uint32_t stage_smem = epi_base + quad * PairCfg<ACC>::EPI_WARP_BYTES;
         uint8_t* stage_ptr = smem_raw + (stage_smem - smem_u32(smem_raw));
         int buf = 0, stores_in_flight = 0;
-        for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-            const PairTile pt = pair_tile(p, tile);
-            const int acc = local_tile & 1;
-            if (!mbar_wait(tfull_bar(acc), acc_phase[acc], &abort_flag)) { ok = false; break; }
-            acc_phase[acc] ^= 1u;
-            tc_fence_after();
-            const int row_w = pt.m0 + static_cast<int>(rank) * 128 + quad * 32;   // first row of this warp
-            const uint32_t t_row = tmem_base + acc * PAIR_BN + (static_cast<uint32_t>(quad * 32) << 16);
+        uint32_t d_phase = 0;      // ACC: parity of each staging tile's next arrival
+        // ACC: request this warp's tiles of D (the stores that last used the staging tiles have finished reading them)
+        auto fetch_d = [&](const PairTile& pt, int row_w) {
+            if (!ACC || row_w >= p.M) return;
+            if (lane == 0) {
+                tma_store_wait_read<0>();
+                for (int i = 0; i < PairCfg<ACC>::EPI_BUFS && pt.n0 + i * 64 < p.N; ++i) {
+                    mbar_expect_tx(d_bar(quad, i), 4096);
+                    tma_load_2d(stage_smem + i * 4096, &tmD, pt.n0 + i * 64, row_w, d_bar(quad, i));
+                }
+            }
+            __syncwarp();
+        };
+        // the finished 32 rows x 256 columns of this warp leave; `load` supplies 32 columns of raw accumulators
+        auto emit = [&](const PairTile& pt, int row_w, auto&& load) {
             if (use_tma_store) {
                 const int cols_per_store = p.out_fp32 ? 32 : 64;
                 if (row_w < p.M) {
 #pragma unroll 1
                     for (int c = 0; c < PAIR_BN && pt.n0 + c < p.N; c += cols_per_store) {
                         uint32_t r0[32], r1[32];
-                        tmem_ld_32x32(t_row + c, r0);
-                        if (!p.out_fp32) tmem_ld_32x32(t_row + c + 32, r1);
-                        if (stores_in_flight >= 2) {      // the store that last read this staging tile has finished reading it
+                        load(c, r0);
+                        if (!p.out_fp32) load(c + 32, r1);
+                        if (ACC) {
+                            buf = c / 64;
+                            if (!mbar_wait(d_bar(quad, buf), (d_phase >> buf) & 1u, &abort_flag)) { ok = false; break; }
+                            d_phase ^= 1u << buf;
+                        } else if (stores_in_flight >= 2) {      // the store that last read this staging tile has finished reading it
                             if (lane == 0) tma_store_wait_read<1>();
                             __syncwarp();
                         }
                         tmem_ld_wait();
                         uint8_t* srow = stage_ptr + buf * 4096 + lane * 128;
-                        if (p.out_fp32) {
+                        if (!ACC && p.out_fp32) {
 #pragma unroll
                             for (int u = 0; u < 8; ++u) {
                                 const float4 v = make_float4(__uint_as_float(r0[u * 4]) * scale, __uint_as_float(r0[u * 4 + 1]) * scale,
@@ -557,27 +676,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         } else {
 #pragma unroll
                             for (int u = 0; u < 8; ++u) {
-                                uint4 o;
+                                uint4* cell = reinterpret_cast<uint4*>(srow + ((u ^ (lane & 7)) << 4));
+                                uint4 o = ACC ? *cell : make_uint4(0, 0, 0, 0);
                                 __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) {
                                     const int e = (u & 3) * 8 + 2 * i;
-                                    const float a = __uint_as_float(u < 4 ? r0[e] : r1[e]) * scale, b = __uint_as_float(u < 4 ? r0[e + 1] : r1[e + 1]) * scale;
+                                    float a = __uint_as_float(u < 4 ? r0[e] : r1[e]) * scale, b = __uint_as_float(u < 4 ? r0[e + 1] : r1[e + 1]) * scale;
+                                    if (ACC) {
+                                        const float2 d = __bfloat1622float2(pb[i]);
+                                        a += d.x;
+                                        b += d.y;
+                                    }
                                     amax = fmaxf(amax, fmaxf(fabsf(a), fabsf(b)));
                                     pb[i] = __floats2bfloat162_rn(a, b);
                                 }
-                                *reinterpret_cast<uint4*>(srow + ((u ^ (lane & 7)) << 4)) = o;
+                                *cell = o;
                             }
                         }
                         fence_proxy_async();
                         __syncwarp();
                         if (lane == 0) {
-                            if (p.accumulate) tma_reduce_add_2d(&tmD, stage_smem + buf * 4096, pt.n0 + c, row_w);
+                            if (!ACC && p.accumulate) tma_reduce_add_2d(&tmD, stage_smem + buf * 4096, pt.n0 + c, row_w);
                             else tma_store_2d(&tmD, stage_smem + buf * 4096, pt.n0 + c, row_w);
                             tma_store_commit();
                         }
                         ++stores_in_flight;
-                        buf ^= 1;
+                        if (!ACC) buf ^= 1;
                     }
                 }
             } else {
@@ -587,16 +712,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 t.d_off = 0;
                 const int row = row_w + lane;
 #pragma unroll 1
-                for (int c = 0; c < PAIR_BN; c += 32) {
+                for (int c = 0; c < PAIR_BN && pt.n0 + c < p.N; c += 32) {
                     uint32_t r[32];
-                    tmem_ld_32x32(t_row + c, r);
+                    load(c, r);
                     tmem_ld_wait();
                     store_direct_32(p, t, row, pt.n0 + c, r, scale, amax);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(tempty_leader[acc]);
+        };
+        for (int unit = first_unit; unit < units && ok; unit += unit_step, ++local_tile) {
+            const Unit u = get_unit(p, num_tiles, num_k, unit);
+            const PairTile pt = pair_tile(p, u.tile);
+            const int acc = local_tile & 1;
+            const int row_w = pt.m0 + static_cast<int>(rank) * 128 + quad * 32;   // first row of this warp
+            const uint32_t t_row = tmem_base + acc * PAIR_BN + (static_cast<uint32_t>(quad * 32) << 16);
+            if (u.piece < 0) fetch_d(pt, row_w);
+            if (!mbar_wait(tfull_bar(acc), acc_phase[acc], &abort_flag)) { ok = false; break; }
+            acc_phase[acc] ^= 1u;
+            tc_fence_after();
+            if (u.piece < 0) {
+                emit(pt, row_w, [&](int c, uint32_t(&r)[32]) { tmem_ld_32x32(t_row + c, r); });
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(tempty_leader[acc]);
+            } else {
+                const int slot = ((u.tile - p.split_from) * 2 + static_cast<int>(rank)) * 4 + quad, slots = (num_tiles - p.split_from) * 8;
+                float4* ws = reinterpret_cast<float4*>(p.workspace) + static_cast<size_t>(slot) * (32 * PAIR_BN / 4);
+                const size_t stride = static_cast<size_t>(slots) * (32 * PAIR_BN / 4);
+                const bool rows = row_w < p.M;
+                if (rows) park_piece<PAIR_BN>(t_row, ws + u.piece * stride, lane, (p.N - pt.n0 + 63) & ~63);   // the reader takes 64 columns at a time
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(tempty_leader[acc]);
+                if (rows && last_piece(p.counters + slot, p.splits, lane)) {
+                    fetch_d(pt, row_w);
+                    emit(pt, row_w, [&](int c, uint32_t(&r)[32]) { sum_pieces(ws, stride, p.splits, lane, c, r); });
+                }
+            }
         }
         if (use_tma_store && lane == 0) tma_store_wait_all();
         if (p.amax_out) {
@@ -668,8 +820,9 @@ template <int BN> static const char* launch(const GemmOperand& A, const GemmOper
             return "cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed";
         attr_set = true;
     }
-    const int num_tiles = p.mode == 0 ? ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) : num_sms;  // grouped: tile count lives on the device
-    const int grid = num_tiles < num_sms ? num_tiles : num_sms;
+    int units = p.mode == 0 ? ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) : num_sms;  // grouped: tile count lives on the device
+    if (p.splits > 1) units = p.split_from + (units - p.split_from) * p.splits;
+    const int grid = units < num_sms ? units : num_sms;
     gemm_tcgen05_kernel<BN><<<grid, GEMM_THREADS, C::SMEM_BYTES, stream>>>(tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? nullptr : "gemm kernel launch failed";
 }
@@ -694,25 +847,88 @@ static const char* launch_pair(const GemmOperand& A, const GemmOperand& B, GemmP
     if (!p.b_mn) e = make_tensor_map_2d(&tmB, B.ptr, p.elem_bytes, p.K, p.N, B.row_stride_bytes, BK, 128);
     else e = make_tensor_map_2d(&tmB, B.ptr, p.elem_bytes, p.N, p.K, B.row_stride_bytes, BK, BK);
     if (e) return e;
-    // The shared-memory epilogue serves plain stores and fp32 accumulation (TMA add).  bf16 accumulation (D is read, summed in
-    // fp32 and rounded once) and an abs-max that must include the accumulated values stay on the register path.
+    // The shared-memory epilogue serves everything but an fp32 abs-max that must include the accumulated values (the TMA add does not
+    // return them).
     const int d_bytes = p.out_fp32 ? 4 : 2;
-    int use_tma_store = (!p.accumulate || (p.out_fp32 && !p.amax_out)) && (static_cast<uint64_t>(p.ldd) * d_bytes) % 16 == 0;
+    int use_tma_store = !(p.accumulate && p.out_fp32 && p.amax_out);
     if (use_tma_store) {
         e = make_tensor_map_2d(&tmD, p.D, d_bytes, p.N, p.M, static_cast<uint64_t>(p.ldd) * d_bytes, 128 / d_bytes, 32);
         if (e) use_tma_store = 0;
     }
     if (!use_tma_store) tmD = tmA;
+    const bool acc = use_tma_store && p.accumulate && !p.out_fp32;
     static bool attr_set = false;
     if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<false>::SMEM_BYTES) != cudaSuccess ||
+            cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<true>::SMEM_BYTES) != cudaSuccess)
             return "cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed (pair GEMM)";
         attr_set = true;
     }
     const int num_tiles = ((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
-    const int clusters = num_tiles < num_sms / 2 ? num_tiles : num_sms / 2;
-    gemm_pair_kernel<<<2 * clusters, GEMM_THREADS, PAIR_SMEM_BYTES, stream>>>(tmA, tmB, tmD, p, use_tma_store);
+    const int units = p.splits > 1 ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
+    const int clusters = units < num_sms / 2 ? units : num_sms / 2;
+    if (acc) gemm_pair_kernel<true><<<2 * clusters, GEMM_THREADS, PairCfg<true>::SMEM_BYTES, stream>>>(tmA, tmB, tmD, p, use_tma_store);
+    else gemm_pair_kernel<false><<<2 * clusters, GEMM_THREADS, PairCfg<false>::SMEM_BYTES, stream>>>(tmA, tmB, tmD, p, use_tma_store);
     return cudaGetLastError() == cudaSuccess ? nullptr : "pair gemm kernel launch failed";
+}
+
+// ------------------------------------------------------------------------------------------------ choice of kernel and split
+// Which kernel runs a dense problem, and into how many pieces the contraction of its last wave of tiles is cut, by estimated time.  The
+// constants are measured (B200, both element widths: a contraction block is 128 bytes deep): one block costs a CTA pair 0.46 us and a
+// single CTA with its 128 x 128 tile 0.36 us; a piece costs its trip through the workspace, its reader all pieces of the tile, and the
+// cleared counters a launch.
+//   pair   : full rate, but 74 tiles of 256 x 256 to a wave.  [1024, 3072] = 16384 deep (48 tiles) in three pieces 164 -> 93 us, [6144, 1024] (96
+//            tiles, the last 22 in three pieces) 204 -> 157 us, [4096, 4096] = 151936 deep in bf16 (256 tiles, 34 in two) 4530 -> 3939 us.
+//   single : four times as many tiles, for small outputs; also the narrow ones (N <= 128), where a pair would multiply padding:
+//            [4096, 16] = 17408 deep 91 -> 45 us in four pieces.
+namespace {
+struct Shape {
+    int tiles, slots;                          // output tiles, tiles that run at once
+    float block_us, piece_us, reader_us;       // per contraction block; per piece of a split tile; per piece for the warp that adds them
+    float split_us;                            // once per split problem
+    int tile_floats;
+};
+struct Split {
+    float us;
+    int from, pieces;
+};
+constexpr int MAX_PIECES = 8;
+constexpr int MIN_PIECE_BLOCKS = 4;
+
+Split best_split(const Shape& h, int num_k) {
+    const int rest = h.tiles % h.slots;
+    const float full = static_cast<float>(h.tiles / h.slots) * num_k * h.block_us;
+    Split best{full + (rest ? num_k * h.block_us : 0.f), h.tiles, 1};
+    for (int s = 2; rest && s <= MAX_PIECES && num_k / s >= MIN_PIECE_BLOCKS && rest * s <= 3 * h.slots; ++s) {
+        const int waves = (rest * s + h.slots - 1) / h.slots;
+        const float us = full + waves * (((num_k + s - 1) / s) * h.block_us + h.piece_us) + s * h.reader_us + h.split_us;
+        if (us < best.us * 0.97f) best = Split{us, h.tiles - rest, s};
+    }
+    return best;
+}
+}  // namespace
+
+GemmPlan gemm_plan_sm100(const GemmParams& p, int num_sms) {
+    GemmPlan plan{0, 1, 0, 0, 0};
+    if (p.mode != 0 || p.M <= 0 || p.N <= 0 || p.K <= 0) return plan;
+    const int num_k = (p.K * p.elem_bytes + TILE_K_BYTES - 1) / TILE_K_BYTES;
+    auto up = [](int a, int b) { return (a + b - 1) / b; };
+    const Shape pair{up(p.M, PAIR_BM) * up(p.N, PAIR_BN), num_sms / 2, 0.46f, 3.0f, 2.5f, 5.0f, PAIR_BM * PAIR_BN};
+    const Shape single{up(p.M, BM) * up(p.N, 128), num_sms, 0.36f, 1.5f, 1.2f, 4.0f, BM * 128};
+    const Split sp = best_split(pair, num_k), ss = best_split(single, num_k);
+    int use_pair = p.tile_n == 512 || (p.tile_n == 0 && p.N > 128 && p.M > 128 && sp.us <= ss.us);
+    plan.pair = use_pair;
+    if (p.tile_n == 256 || p.tile_n == 128) return plan;        // forced single-CTA tiles: never split
+    const Split& c = use_pair ? sp : ss;
+    if (c.pieces > 1) {
+        const Shape& h = use_pair ? pair : single;
+        const size_t cut = static_cast<size_t>(h.tiles - c.from);
+        plan.splits = c.pieces;
+        plan.split_from = c.from;
+        plan.workspace_floats = cut * c.pieces * h.tile_floats;
+        plan.num_counters = cut * (use_pair ? 8 : 4);
+    }
+    return plan;
 }
 
 const char* gemm_sm100(const GemmOperand& A, const GemmOperand& B, GemmParams p, int num_sms, cudaStream_t stream) {
@@ -720,13 +936,18 @@ const char* gemm_sm100(const GemmOperand& A, const GemmOperand& B, GemmParams p,
     if (p.mode != 0 && (p.num_groups <= 0 || p.num_groups > MAX_GROUPS || !p.group_offsets)) return "gemm_sm100: grouped mode needs 1..256 groups and offsets";
     if (p.N % 8 != 0 || p.ldd % 8 != 0) return "gemm_sm100: N and ldd must be multiples of 8";
     if ((reinterpret_cast<uintptr_t>(p.D) & 15) != 0) return "gemm_sm100: D must be 16-byte aligned";
-    // CTA pairs (256 x 256 per cluster) for dense problems with at least one tile per cluster; tile_n = 512 forces them, 128 / 256
-    // force the single-CTA kernels
-    const long tiles_pair = static_cast<long>((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
-    if (p.mode == 0 && (p.tile_n == 512 || (p.tile_n == 0 && tiles_pair >= num_sms / 2))) return launch_pair(A, B, p, num_sms, stream);
+    const GemmPlan plan = gemm_plan_sm100(p, num_sms);
+    if (p.workspace && p.counters) {        // a caller without them gets the same kernel, unsplit
+        p.splits = plan.splits;
+        p.split_from = plan.split_from;
+        if (plan.splits > 1 && cudaMemsetAsync(p.counters, 0, plan.num_counters * sizeof(int), stream) != cudaSuccess) return "gemm_sm100: clearing the counters failed";
+    } else {
+        p.splits = 1;
+    }
+    if (plan.pair) return launch_pair(A, B, p, num_sms, stream);
     // 128-wide N tiles when the wide tile would leave SMs idle or N is small
     const long tiles256 = static_cast<long>((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
-    const bool narrow = p.N <= 128 || (p.tile_n == 128) || (p.tile_n == 0 && tiles256 < num_sms);
+    const bool narrow = p.mode == 0 ? p.tile_n != 256 : p.N <= 128 || (p.tile_n == 128) || (p.tile_n == 0 && tiles256 < num_sms);
     return narrow ? launch<128>(A, B, p, num_sms, stream) : launch<256>(A, B, p, num_sms, stream);
 }
 

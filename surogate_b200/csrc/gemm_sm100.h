@@ -36,7 +36,18 @@ struct GemmParams {
     const int* group_offsets;    // device, num_groups + 1 entries
     long long a_total_rows;      // stored rows of A (grouped modes)
     long long b_total_rows;      // stored rows of B (grouped modes)
+    // Split contraction (dense problems): the caller sizes these with gemm_plan_sm100; both null = no split.
+    float* workspace;            // plan.workspace_floats, 16-byte aligned, any content
+    int* counters;               // plan.num_counters, cleared by the launch
+    int splits, split_from;      // set by gemm_sm100
 };
+
+// How a dense problem will run: CTA pairs or single CTAs, and the pieces that the contraction of tiles split_from.. is cut into.
+struct GemmPlan {
+    int pair, splits, split_from;
+    size_t workspace_floats, num_counters;
+};
+GemmPlan gemm_plan_sm100(const GemmParams& p, int num_sms);
 
 const char* gemm_sm100(const GemmOperand& A, const GemmOperand& B, GemmParams p, int num_sms, cudaStream_t stream);
 

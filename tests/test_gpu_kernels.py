@@ -97,6 +97,67 @@ def test_gemm_cta_pair(ext, M, N, K, a_mn, b_mn, fp8):
     _check_flag()
 
 
+SPLIT_SHAPES = [(16, 5120, 4096, 0), (1024, 16, 8192, 0), (136, 200, 2056, 0),     # single CTAs, every tile cut
+                (1024, 1024, 6144, 512), (3000, 1000, 4104, 0),                     # CTA pairs, every tile cut, ragged edges
+                (2560, 2048, 2112, 512), (5376, 1032, 1536, 512)]                   # whole waves, then cut tiles
+
+
+@pytest.mark.parametrize("M,N,K,tile_n", SPLIT_SHAPES)
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_gemm_with_a_split_contraction(ext, M, N, K, tile_n, a_mn, b_mn, fp8):
+    """Shapes whose tiles leave SMs idle are cut along the contraction.  bf16 and fp32 outputs, plain and accumulated, against fp32
+    PyTorch: the error is the rounding of the output (2^-9 per element, twice with accumulation) and of fp32 sums; and the same bits twice,
+    since the pieces are added in a fixed order."""
+    from surogate_b200.runtime.ops_cuda import gemm
+
+    es = 1 if fp8 else 2
+    if (a_mn and M * es % 16) or (b_mn and N * es % 16) or K * es % 16:
+        pytest.skip("row stride must be a multiple of 16 bytes")
+    torch.manual_seed(M + N + K)
+    dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device=DEV).to(dt)
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device=DEV).to(dt)
+    ref = (a.float().t() if a_mn else a.float()) @ (b.float() if b_mn else b.float().t())
+    D0 = torch.randn(M, N, device=DEV) * K ** 0.5
+    wide = torch.zeros(M, N + 24, device=DEV, dtype=torch.bfloat16)      # a strided output: nothing outside it may change
+    out = wide[:, 8:8 + N]
+    gemm(a, b, out, a_mn=a_mn, b_mn=b_mn, tile_n=tile_n)
+    again = gemm(a, b, a_mn=a_mn, b_mn=b_mn, tile_n=tile_n)
+    acc = D0.bfloat16()
+    amax = torch.zeros(1, device=DEV)
+    gemm(a, b, acc, a_mn=a_mn, b_mn=b_mn, tile_n=tile_n, accumulate=True, alpha=0.5, amax_out=amax)
+    acc32 = D0.clone()
+    gemm(a, b, acc32, a_mn=a_mn, b_mn=b_mn, tile_n=tile_n, accumulate=True, alpha=0.5)
+    torch.cuda.synchronize()
+    _check_flag()
+    assert torch.equal(out, again) and not wide[:, :8].any() and not wide[:, 8 + N:].any()
+    assert _rel_err(out, ref) < 2.5e-3
+    want = D0.bfloat16().float() + 0.5 * ref
+    assert _rel_err(acc, want) < 2.5e-3
+    assert abs(amax.item() - acc.float().abs().max().item()) <= 2 ** -8 * amax.item()
+    assert _rel_err(acc32, D0 + 0.5 * ref) < 2e-5
+
+
+def test_gemm_bf16_accumulation_with_a_short_contraction(ext):
+    """D += A.B^T where D is the traffic (adapter updates, gradient accumulation): its tiles travel through shared memory both ways."""
+    from surogate_b200.runtime.ops_cuda import gemm
+
+    torch.manual_seed(3)
+    for M, N, K in [(8192, 4096, 16), (4000, 5128, 48), (2600, 2056, 72)]:
+        h = torch.randn(M, 3 * K, device=DEV).bfloat16()
+        a, b = h[:, K:2 * K], torch.randn(N, K, device=DEV).bfloat16()
+        wide = torch.randn(M, N + 64, device=DEV).bfloat16()
+        before = wide.clone()
+        gemm(a, b, wide[:, 32:32 + N], accumulate=True, alpha=2.0)
+        torch.cuda.synchronize()
+        _check_flag()
+        want = before[:, 32:32 + N].float() + 2.0 * (a.float() @ b.float().t())
+        assert (wide[:, 32:32 + N].float() - want).abs().max() <= 2 ** -8 * want.abs().max()
+        assert _rel_err(wide[:, 32:32 + N], want) < 2.5e-3
+        assert torch.equal(wide[:, :32], before[:, :32]) and torch.equal(wide[:, 32 + N:], before[:, 32 + N:])
+
+
 def test_gemm_accumulate_fp32_and_alpha(ext):
     from surogate_b200.runtime.ops_cuda import gemm
 
