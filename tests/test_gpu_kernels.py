@@ -374,6 +374,17 @@ def test_quantize_fp8_and_sumsq(ext):
     assert abs(ext.sumsq(xf).item() / xf.pow(2).sum().item() - 1) < 1e-5
 
 
+@pytest.mark.parametrize("shape", [(1, 8), (3, 40), (129, 1000), (2, 3, 48), (4096, 272)])
+@pytest.mark.parametrize("dt", [torch.float8_e4m3fn, torch.float8_e5m2])
+def test_dequantize_fp8(ext, shape, dt):
+    """Counts below, at and off the 16 values of a thread: the fp32 product rounded once, so the bits are PyTorch's."""
+    torch.manual_seed(sum(shape))
+    q = (torch.randn(*shape, device=DEV) * 20).to(dt)
+    scale = torch.tensor([0.0371], device=DEV)
+    out = ext.dequantize_fp8(q, scale)
+    assert out.shape == q.shape and torch.equal(out, (q.float() * scale).bfloat16())
+
+
 def test_adamw_kernels(ext):
     n = 100000 - 100000 % 32
     p = torch.randn(n, device=DEV)
