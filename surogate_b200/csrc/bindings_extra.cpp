@@ -421,11 +421,11 @@ Tensor flash_attn_fwd_profile(const Tensor& qkv, int64_t Hq, int64_t Hkv, double
 Tensor flash_attn_bwd_profile(const Tensor& d_out, const Tensor& qkv, const Tensor& lse, int64_t Hq, int64_t Hkv, double scale) {
     const int B = static_cast<int>(qkv.size(0)), T = static_cast<int>(qkv.size(1));
     Tensor d_qkv = torch::empty_like(qkv);
-    Tensor delta = torch::zeros_like(lse);
+    Tensor stats = torch::empty({2 * lse.numel()}, lse.options());
     Tensor prof = torch::zeros({16}, qkv.options().dtype(at::kLong));
-    const char* err = sg::flash_attn_bwd64_sm100(qkv.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(), d_qkv.data_ptr(), B, T,
-                                                 static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<float>(scale), sg_error_flag(), cur_stream(),
-                                                 reinterpret_cast<long long*>(prof.data_ptr<int64_t>()));
+    const char* err = sg::flash_attn_bwd_sm100(qkv.data_ptr(), d_out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), stats.data_ptr<float>(), d_qkv.data_ptr(),
+                                               B, T, static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<float>(scale), sg_error_flag(), sms(), cur_stream(),
+                                               nullptr, nullptr, reinterpret_cast<long long*>(prof.data_ptr<int64_t>()));
     TORCH_CHECK(err == nullptr, err ? err : "");
     return prof;
 }
@@ -439,6 +439,11 @@ Tensor flash_attn_bwd(const Tensor& d_out, const Tensor& qkv, const Tensor& out,
     const int B = static_cast<int>(qkv.size(0)), T = static_cast<int>(qkv.size(1));
     const c10::cuda::CUDAGuard guard(qkv.device());
     const int* lo_p = lo_ptr(lo, qkv);
+    Tensor lo_copy;
+    if (lo_p && (reinterpret_cast<uintptr_t>(lo_p) & 15) != 0) {   // the kernel copies 16 bytes at a time
+        lo_copy = lo->clone();
+        lo_p = lo_copy.data_ptr<int>();
+    }
     const int* qend_p = nullptr;
     if (lo_p) {
         TORCH_CHECK(kv_qend.has_value() && kv_qend->is_cuda() && kv_qend->scalar_type() == at::kInt && kv_qend->is_contiguous() &&
@@ -447,9 +452,9 @@ Tensor flash_attn_bwd(const Tensor& d_out, const Tensor& qkv, const Tensor& out,
         qend_p = kv_qend->data_ptr<int>();
     }
     Tensor d_qkv = torch::empty_like(qkv);
-    Tensor delta = torch::empty_like(lse);
+    Tensor stats = torch::empty({2 * lse.numel()}, lse.options());
     sg_count_launch(3);
-    const char* err = sg::flash_attn_bwd_sm100(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
+    const char* err = sg::flash_attn_bwd_sm100(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), stats.data_ptr<float>(),
                                                d_qkv.data_ptr(), B, T, static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<float>(scale),
                                                sg_error_flag(), sms(), cur_stream(), lo_p, qend_p);
     TORCH_CHECK(err == nullptr, err ? err : "");

@@ -126,6 +126,15 @@ def test_flash_attention_packed_documents_and_windows(B, T, Hq, Hkv, window, doc
     _check_bwd(qkv, Hq, Hkv, bounds)
 
 
+@pytest.mark.parametrize("B,T,Hq,Hkv,window", [(1, 128, 3, 1, 0), (1, 384, 3, 1, 0), (3, 640, 10, 2, 0), (2, 896, 5, 5, 0), (1, 384, 3, 1, 3), (2, 640, 6, 2, 100)])   # a window of one has dq = 0: no relative error
+def test_flash_attention_backward_item_counts(B, T, Hq, Hkv, window):
+    """The two groups of softmax warps take alternate 64-row items through a ring of four: item counts from one or two per CTA (one group
+    idle, the ring never wraps) to many, even and odd, with three and five query heads per KV head."""
+    torch.manual_seed(B * T + Hq + window)
+    qkv = torch.randn(B, T, (Hq + 2 * Hkv) * D, device=DEV).bfloat16()
+    _check_bwd(qkv, Hq, Hkv, _packed_lo(B, T, window, False) if window else None)
+
+
 def test_packed_batch_trains_like_the_masked_fp32_path():
     """One packed batch (position ids reset inside the rows) and one sliding-window model through the trainer on the CUDA backend:
     loss and gradient norm equal the PyTorch backend, whose attention applies the explicit document / window mask."""
