@@ -459,6 +459,30 @@ def test_adamw_8bit_kernel_matches_the_pytorch_twin_code_for_code(ext):
 
 
 # ----------------------------------------------------------------------------- MoE
+@pytest.mark.parametrize("n", [32, 2048, 2080, 148 * 3 * 256 * 8 + 32, 148 * 3 * 256 * 8 * 5 + 160])
+@pytest.mark.parametrize("pdt,gdt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
+def test_adamw_8bit_counts(ext, n, pdt, gdt):
+    """Counts from part of a warp to several trips around the shared-memory ring: every element is updated once, as when the same values
+    are stepped in pieces of 32 (groups of 32 share a scale, so the pieces do not interact)."""
+    torch.manual_seed(n % 997)
+    hp = torch.tensor([1e-2, 0.9, 0.99, 1e-8, 0.1, 0.1, 0.01, 0.5], device=DEV)
+    p, g = torch.randn(n, device=DEV).to(pdt), torch.randn(n, device=DEV).to(gdt)
+
+    def state(k):
+        return [torch.zeros(k, dtype=torch.int8, device=DEV), torch.zeros(k, dtype=torch.uint8, device=DEV),
+                torch.zeros(k // 32, dtype=torch.float16, device=DEV), torch.zeros(k // 32, dtype=torch.float16, device=DEV)]
+
+    full, st = p.clone(), state(n)
+    for _ in range(2):
+        ext.adamw8_step(full, g, *st, None, hp)
+    for lo in sorted({0, n // 64 * 32, n - 32}):
+        part, ps = p[lo:lo + 32].clone(), state(32)
+        for _ in range(2):
+            ext.adamw8_step(part, g[lo:lo + 32].clone(), *ps, None, hp)
+        assert torch.equal(full[lo:lo + 32], part) and torch.equal(st[0][lo:lo + 32], ps[0]) and torch.equal(st[3][lo // 32:lo // 32 + 1], ps[3])
+    assert not torch.equal(full, p) and (full != p).float().mean().item() > 0.9
+
+
 def test_moe_softmax_topk(ext):
     tokens, E, K = 1000, 128, 8
     logits = torch.randn(tokens, E, device=DEV)
