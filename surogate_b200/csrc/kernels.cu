@@ -61,57 +61,105 @@ template <bool IS_MAX> __device__ __forceinline__ float block_reduce(float v, fl
 __device__ __forceinline__ void atomic_max_pos(float* addr, float v) {
     if (v > 0.f) atomicMax(reinterpret_cast<unsigned int*>(addr), __float_as_uint(v));
 }
-template <bool E5M2> __device__ __forceinline__ uint8_t to_fp8(float v) {
-    return E5M2 ? __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E5M2) : __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+
+// eight values times `s` as FP8, two to a conversion instruction
+template <bool E5M2> __device__ __forceinline__ uint2 to_fp8x8(const float (&a)[8], float s) {
+    uint2 o;
+    __nv_fp8x2_storage_t* ob = reinterpret_cast<__nv_fp8x2_storage_t*>(&o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ob[i] = __nv_cvt_float2_to_fp8x2(make_float2(a[2 * i] * s, a[2 * i + 1] * s), __NV_SATFINITE, E5M2 ? __NV_E5M2 : __NV_E4M3);
+    return o;
 }
 
 // ------------------------------------------------------------------------------------------ RMSNorm forward
-// one CTA per row.  res_out = residual + x (optional) ; y = res_out * rstd * w ; optionally y also as FP8.
+// One CTA per row.  res_out = residual + x (optional) ; y = res_out * rstd * w ; optionally y also as FP8.
+// ITERS > 0: the row (C <= blockDim * 8 * ITERS) stays in registers as packed bf16 between the sum and the scaling, with all its loads and
+// those of w in flight together; ITERS = 0 (wider rows) reads it again.
+// With the residual on B200: 16384 x 1024 37 -> 27 us, 8192 x 4096 64 -> 48 us (FP8 output 60 -> 44), 8192 x 5120 78 -> 64 us.
+template <int ITERS>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, const bf16* __restrict__ w,
                                                           bf16* __restrict__ res_out, bf16* __restrict__ y, float* __restrict__ rstd_out,
                                                           uint8_t* __restrict__ y_fp8, const float* __restrict__ fp8_scale, float* __restrict__ amax_out,
                                                           int C, float eps) {
     __shared__ float sh[32];
+    constexpr int N = ITERS > 0 ? ITERS : 1;
     const size_t row = blockIdx.x;
     const bf16* xr = x + row * C;
     const bf16* rr = residual ? residual + row * C : nullptr;
     bf16* ro = res_out ? res_out + row * C : nullptr;
+    const int step = blockDim.x * 8;
     float ss = 0.f;
-    for (int c = threadIdx.x * 8; c < C; c += blockDim.x * 8) {
-        float a[8];
-        load8(xr + c, a);
-        if (rr) {
-            float b[8];
-            load8(rr + c, b);
+    uint4 xk[N], rk[N], wk[N];
+    auto add_residual = [&](uint4 xv, uint4 rv) {   // rounded to the stored precision, so that forward and backward see the same residual stream
+        float a[8], b[8];
+        unpack8(xv, a);
+        unpack8(rv, b);
+        uint4 o;
+        bf162* po = reinterpret_cast<bf162*>(&o);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] += b[i];
-            // round to the stored precision so forward and backward see the same residual stream
-            store8(ro + c, a);
-            load8(ro + c, a);
-        }
+        for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(a[2 * i] + b[2 * i], a[2 * i + 1] + b[2 * i + 1]);
+        return o;
+    };
+    auto square = [&](const uint4& v) {
+        float a[8];
+        unpack8(v, a);
 #pragma unroll
         for (int i = 0; i < 8; ++i) ss += a[i] * a[i];
+    };
+    if (ITERS > 0) {
+#pragma unroll
+        for (int it = 0; it < N; ++it) {
+            const int c = threadIdx.x * 8 + it * step;
+            if (c < C) {
+                xk[it] = *reinterpret_cast<const uint4*>(xr + c);
+                if (rr) rk[it] = *reinterpret_cast<const uint4*>(rr + c);
+                wk[it] = *reinterpret_cast<const uint4*>(w + c);
+            }
+        }
+#pragma unroll
+        for (int it = 0; it < N; ++it) {
+            const int c = threadIdx.x * 8 + it * step;
+            if (c < C) {
+                if (rr) {
+                    xk[it] = add_residual(xk[it], rk[it]);
+                    *reinterpret_cast<uint4*>(ro + c) = xk[it];
+                }
+                square(xk[it]);
+            }
+        }
+    } else {
+        for (int c = threadIdx.x * 8; c < C; c += step) {
+            uint4 v = *reinterpret_cast<const uint4*>(xr + c);
+            if (rr) {
+                v = add_residual(v, *reinterpret_cast<const uint4*>(rr + c));
+                *reinterpret_cast<uint4*>(ro + c) = v;
+            }
+            square(v);
+        }
     }
     ss = block_reduce<false>(ss, sh);
     const float rstd = rsqrtf(ss / C + eps);
     if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-    const bf16* src = rr ? ro : xr;
     const float qs = fp8_scale ? __ldg(fp8_scale) : 1.f;
     float amax = 0.f;
-    for (int c = threadIdx.x * 8; c < C; c += blockDim.x * 8) {
+    auto scale_out = [&](int c, const uint4& v, const uint4& wv) {
         float a[8], g[8];
-        load8(src + c, a);
-        load8(w + c, g);
+        unpack8(v, a);
+        unpack8(wv, g);
 #pragma unroll
         for (int i = 0; i < 8; ++i) { a[i] = a[i] * rstd * g[i]; amax = fmaxf(amax, fabsf(a[i])); }
         if (y) store8(y + row * C + c, a);
-        if (y_fp8) {
-            uint2 o;
-            uint8_t* ob = reinterpret_cast<uint8_t*>(&o);
+        if (y_fp8) *reinterpret_cast<uint2*>(y_fp8 + row * C + c) = to_fp8x8<false>(a, qs);
+    };
+    if (ITERS > 0) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ob[i] = to_fp8<false>(a[i] * qs);
-            *reinterpret_cast<uint2*>(y_fp8 + row * C + c) = o;
+        for (int it = 0; it < N; ++it) {
+            const int c = threadIdx.x * 8 + it * step;
+            if (c < C) scale_out(c, xk[it], wk[it]);
         }
+    } else {
+        const bf16* src = rr ? ro : xr;
+        for (int c = threadIdx.x * 8; c < C; c += step) scale_out(c, *reinterpret_cast<const uint4*>(src + c), *reinterpret_cast<const uint4*>(w + c));
     }
     if (amax_out) {
         amax = block_reduce<true>(amax, sh);
@@ -261,13 +309,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict_
 #pragma unroll
             for (int i = 0; i < 8; ++i) { o[i] = gate[i] / (1.f + __expf(-gate[i])) * up[i]; amax = fmaxf(amax, fabsf(o[i])); }
             if (y) store8(y + row * M + c, o);
-            if (y_fp8) {
-                uint2 q;
-                uint8_t* qb = reinterpret_cast<uint8_t*>(&q);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) qb[i] = to_fp8<false>(o[i] * qs);
-                *reinterpret_cast<uint2*>(y_fp8 + row * M + c) = q;
-            }
+            if (y_fp8) *reinterpret_cast<uint2*>(y_fp8 + row * M + c) = to_fp8x8<false>(o, qs);
         }
     }
     if (amax_out) {
@@ -301,17 +343,10 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict_
             store8(dx + row * 2 * M + M + c, dg);
         }
         if (dx_fp8) {
-            uint2 qu, qg;
-            uint8_t* bu = reinterpret_cast<uint8_t*>(&qu);
-            uint8_t* bg = reinterpret_cast<uint8_t*>(&qg);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                amax = fmaxf(amax, fmaxf(fabsf(du[i]), fabsf(dg[i])));
-                bu[i] = to_fp8<true>(du[i] * qs);
-                bg[i] = to_fp8<true>(dg[i] * qs);
-            }
-            *reinterpret_cast<uint2*>(dx_fp8 + row * 2 * M + c) = qu;
-            *reinterpret_cast<uint2*>(dx_fp8 + row * 2 * M + M + c) = qg;
+            for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fmaxf(fabsf(du[i]), fabsf(dg[i])));
+            *reinterpret_cast<uint2*>(dx_fp8 + row * 2 * M + c) = to_fp8x8<true>(du, qs);
+            *reinterpret_cast<uint2*>(dx_fp8 + row * 2 * M + M + c) = to_fp8x8<true>(dg, qs);
         }
     }
     if (amax_out) {
@@ -659,11 +694,9 @@ __global__ void __launch_bounds__(256) quantize_fp8_kernel(const bf16* __restric
     for (size_t v = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; v < nvec; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float a[8];
         load8(x + v * 8, a);
-        uint2 o;
-        uint8_t* ob = reinterpret_cast<uint8_t*>(&o);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { amax = fmaxf(amax, fabsf(a[i])); ob[i] = to_fp8<E5M2>(a[i] * s); }
-        *reinterpret_cast<uint2*>(q + v * 8) = o;
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(a[i]));
+        *reinterpret_cast<uint2*>(q + v * 8) = to_fp8x8<E5M2>(a, s);
     }
     if (amax_out) {
         amax = block_reduce<true>(amax, sh);
@@ -974,8 +1007,15 @@ void rmsnorm_fwd(const void* x, const void* residual, const void* w, void* res_o
                  float* amax, int rows, int C, float eps, cudaStream_t s) {
     int threads = C / 8;
     threads = threads > 256 ? 256 : (threads < 32 ? 32 : (threads + 31) / 32 * 32);
-    rmsnorm_fwd_kernel<<<rows, threads, 0, s>>>((const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)res_out, (bf16*)y, rstd, (uint8_t*)y_fp8,
-                                                fp8_scale, amax, C, eps);
+    const int iters = (C + threads * 8 - 1) / (threads * 8);
+#define SG_RF(IT)                                                                                                                              \
+    rmsnorm_fwd_kernel<IT><<<rows, threads, 0, s>>>((const bf16*)x, (const bf16*)residual, (const bf16*)w, (bf16*)res_out, (bf16*)y, rstd,     \
+                                                    (uint8_t*)y_fp8, fp8_scale, amax, C, eps)
+    if (iters <= 1) SG_RF(1);
+    else if (iters <= 2) SG_RF(2);
+    else if (iters <= 4) SG_RF(4);
+    else SG_RF(0);
+#undef SG_RF
 }
 int rmsnorm_bwd_blocks(int rows, int num_sms) { return rows < num_sms * 2 ? rows : num_sms * 2; }
 static int rmsnorm_bwd_threads(int C) { return C <= 1024 ? 128 : RB_THREADS; }

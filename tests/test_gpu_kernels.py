@@ -248,6 +248,60 @@ def test_rmsnorm_weight_gradient_sums(ext, rows, C):
     assert torch.equal(dw, ext.rmsnorm_bwd(dy, x, w, rstd, None)[1])
 
 
+@pytest.mark.parametrize("rows,C", [(1, 8), (3, 256), (5, 2048), (4, 2056), (3, 4096), (2, 8192), (2, 8200)])
+def test_rmsnorm_forward_widths(ext, rows, C):
+    """Widths around those at which the row is kept in one, two or four vectors per thread, and beyond."""
+    torch.manual_seed(C)
+    x, res, w = (torch.randn(*s, device=DEV).bfloat16() for s in ((rows, C), (rows, C), (C,)))
+    r, y, rstd, _ = ext.rmsnorm_fwd(x, res, w, 1e-6, True, None, None, False)
+    scale, amax = torch.tensor([3.0], device=DEV), torch.zeros(1, device=DEV)
+    _, _, _, y8 = ext.rmsnorm_fwd(x, res, w, 1e-6, False, scale, amax, True)
+    want_r = x + res
+    want = want_r.float() * torch.rsqrt(want_r.float().pow(2).mean(-1, keepdim=True) + 1e-6) * w.float()
+    assert torch.equal(r, want_r) and _rel_err(y, want) < 3e-3          # one bf16 rounding
+    assert _rel_err(y8.float() / 3.0, want) < 4e-2                      # one E4M3 rounding
+    assert abs(amax.item() - want.abs().max().item()) < 1e-4 * amax.item()
+    y0 = ext.rmsnorm_fwd(x, None, w, 1e-6, True, None, None, False)[1]
+    want0 = x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-6) * w.float()
+    assert _rel_err(y0, want0) < 3e-3
+
+
+@pytest.mark.parametrize("rows,M", [(1, 8), (3, 264), (2, 12288), (8193, 768), (1025, 2056)])
+def test_swiglu_row_counts(ext, rows, M):
+    """Row counts that leave the second row of a thread's pair behind the end, and one row."""
+    torch.manual_seed(rows + M)
+    x, dy = torch.randn(rows, 2 * M, device=DEV).bfloat16(), torch.randn(rows, M, device=DEV).bfloat16()
+    xr = x.float().requires_grad_(True)
+    ref = torch.nn.functional.silu(xr[:, M:]) * xr[:, :M]
+    ref.backward(dy.float())
+    scale, amax = torch.tensor([2.0], device=DEV), torch.zeros(1, device=DEV)
+    y, y8 = ext.swiglu_fwd(x, True, scale, amax, True)
+    assert _rel_err(y, ref.detach()) < 3e-3 and _rel_err(y8.float() / 2.0, ref.detach()) < 4e-2
+    assert abs(amax.item() - ref.abs().max().item()) < 1e-3 * amax.item()
+    assert _rel_err(ext.swiglu_bwd(dy, x), xr.grad) < 3e-3
+    d8 = ext.swiglu_bwd_fp8(dy, x, scale, torch.zeros(1, device=DEV))
+    assert _rel_err(d8.float() / 2.0, xr.grad) < 8e-2                   # one E5M2 rounding
+    limit = torch.tensor([rows // 2], device=DEV, dtype=torch.int32)
+    half = ext.swiglu_fwd(x, True, None, None, False, limit)[0]
+    assert torch.equal(half[:rows // 2], y[:rows // 2])
+
+
+@pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
+@pytest.mark.parametrize("e5m2", [False, True])
+def test_quantize_fp8_counts(ext, n, e5m2):
+    """Counts at which a thread has no, one, some or all of its four vectors: the bits of PyTorch's conversion (saturating), and the abs-max."""
+    torch.manual_seed(n % 1000)
+    x = (torch.randn(n, device=DEV) * 200).bfloat16()
+    x[-1] = -3000.0
+    scale, amax, amax2 = torch.tensor([1.7], device=DEV), torch.zeros(1, device=DEV), torch.zeros(1, device=DEV)
+    q = ext.quantize_fp8(x, scale, amax, e5m2)
+    dt, top = (torch.float8_e5m2, 57344.0) if e5m2 else (torch.float8_e4m3fn, 448.0)
+    want = (x.float() * scale).clamp(-top, top).to(dt)
+    assert torch.equal(q.view(torch.uint8), want.view(torch.uint8)) and amax.item() == x.float().abs().max().item()
+    ext.amax(x, amax2)
+    assert amax2.item() == amax.item()
+
+
 def test_swiglu(ext):
     rows, M = 517, 3072
     x = torch.randn(rows, 2 * M, device=DEV).bfloat16()
