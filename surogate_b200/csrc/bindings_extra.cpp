@@ -164,6 +164,23 @@ void moe_permute(const Tensor& x, const Tensor& topk_idx, const Tensor& offsets,
                     tokens, C, K, static_cast<int>(expert_base), static_cast<int>(num_local), static_cast<int>(xp.size(0)), cur_stream());
 }
 
+// Zeroes the rows of an expert buffer behind offsets[E] and, with `counts`, the padding of each group.
+void moe_zero_rows(Tensor& buf, const Tensor& offsets, const c10::optional<Tensor>& counts) {
+    TORCH_CHECK(buf.is_cuda() && buf.is_contiguous() && buf.dim() == 2, "moe_zero_rows: a contiguous CUDA matrix");
+    const int64_t row_bytes = buf.size(1) * buf.element_size();
+    TORCH_CHECK(row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(buf.data_ptr()) & 15) == 0, "moe_zero_rows: rows of whole 16-byte vectors");
+    TORCH_CHECK(offsets.is_cuda() && offsets.scalar_type() == at::kInt && offsets.is_contiguous() && offsets.numel() >= 2, "offsets: CUDA int32 [E + 1]");
+    const int E = static_cast<int>(offsets.numel()) - 1;
+    const int* c = nullptr;
+    if (counts.has_value() && counts->defined()) {
+        TORCH_CHECK(counts->is_cuda() && counts->scalar_type() == at::kInt && counts->is_contiguous() && counts->numel() == E, "counts: CUDA int32 [E]");
+        c = counts->data_ptr<int>();
+    }
+    const c10::cuda::CUDAGuard guard(buf.device());
+    sg_count_launch(1);
+    sg::moe_zero_rows(buf.data_ptr(), offsets.data_ptr<int>(), c, E, static_cast<int>(row_bytes), static_cast<int>(buf.size(0)), sms(), cur_stream());
+}
+
 Tensor moe_unpermute(const Tensor& yp, const c10::optional<Tensor>& w, const Tensor& row_map, int64_t tokens, int64_t K) {
     TORCH_CHECK(yp.scalar_type() == at::kBFloat16 && yp.is_contiguous(), "yp: bf16 contiguous");
     const int C = static_cast<int>(yp.size(-1));
@@ -174,11 +191,15 @@ Tensor moe_unpermute(const Tensor& yp, const c10::optional<Tensor>& w, const Ten
     return y;
 }
 
-std::vector<Tensor> moe_unpermute_bwd(const Tensor& dy, const Tensor& yp, const Tensor& w, const Tensor& row_map) {
+// `offsets` / `counts` of the plan: only the rows that no token owns are cleared in d_yp; without them all of it is.
+std::vector<Tensor> moe_unpermute_bwd(const Tensor& dy, const Tensor& yp, const Tensor& w, const Tensor& row_map, const c10::optional<Tensor>& offsets,
+                                      const c10::optional<Tensor>& counts) {
     TORCH_CHECK(dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && yp.is_contiguous(), "bf16 contiguous");
     const int C = static_cast<int>(yp.size(-1));
     const int tokens = static_cast<int>(dy.numel() / C), K = static_cast<int>(w.size(-1));
-    Tensor d_yp = torch::zeros_like(yp);
+    const bool sparse = offsets.has_value() && offsets->defined() && counts.has_value() && counts->defined() && C % 8 == 0;
+    Tensor d_yp = sparse ? torch::empty_like(yp) : torch::zeros_like(yp);
+    if (sparse) moe_zero_rows(d_yp, *offsets, counts);
     Tensor d_w = torch::empty_like(w);
     sg_count_launch(1);
     sg::moe_unpermute_bwd(dy.data_ptr(), yp.data_ptr(), w.data_ptr<float>(), row_map.data_ptr<int>(), d_yp.data_ptr(), d_w.data_ptr<float>(), tokens, C, K,
@@ -602,7 +623,9 @@ void sg_register_extra(pybind11::module_& m) {
     m.def("moe_offsets", &moe_offsets);
     m.def("moe_permute", &moe_permute);
     m.def("moe_unpermute", &moe_unpermute);
-    m.def("moe_unpermute_bwd", &moe_unpermute_bwd);
+    m.def("moe_zero_rows", &moe_zero_rows, pybind11::arg("buf"), pybind11::arg("offsets"), pybind11::arg("counts") = c10::optional<Tensor>());
+    m.def("moe_unpermute_bwd", &moe_unpermute_bwd, pybind11::arg("dy"), pybind11::arg("yp"), pybind11::arg("w"), pybind11::arg("row_map"),
+          pybind11::arg("offsets") = c10::optional<Tensor>(), pybind11::arg("counts") = c10::optional<Tensor>());
     m.def("gemm_grouped", &gemm_grouped);
     m.def("nvfp4_sf_bytes", &nvfp4_sf_bytes);
     m.def("nvfp4_quantize", &nvfp4_quantize, pybind11::arg("x"), pybind11::arg("amax"), pybind11::arg("stochastic"), pybind11::arg("seed"), pybind11::arg("block2d"),

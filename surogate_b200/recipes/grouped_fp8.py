@@ -124,6 +124,7 @@ class GroupedFp8Mixin:
         if not self._grouped_active(ctx, op, x, w):
             return None
         from ..ops import ext as _ext
+        from ..runtime.ops_cuda import grouped_output
 
         ext = _ext()
         role = op.attrs["role"]
@@ -133,7 +134,7 @@ class GroupedFp8Mixin:
         else:
             x8, x_inv = self._gq(ext, x, False, used, self._gslot(ctx.layer, role, "x"))
         w8, w_inv = self._expert_weight(ctx, ext, role, w)
-        y = (torch.empty if used is not None else torch.zeros)(x.shape[0], w.shape[1], dtype=torch.bfloat16, device=x.device)
+        y = grouped_output(ext, (x.shape[0], w.shape[1]), x, plan, used)
         ext.gemm_grouped(x8, w8, y, plan.offsets, 1, False, False, 1.0, x_inv, w_inv, ext.error_flag_tensor())
         if used is not None:
             y._sg_rows = used
@@ -144,6 +145,7 @@ class GroupedFp8Mixin:
         if not self._grouped_active(ctx, op, x, w):
             return None
         from ..ops import ext as _ext
+        from ..runtime.ops_cuda import grouped_output
 
         ext = _ext()
         err = ext.error_flag_tensor()
@@ -153,7 +155,7 @@ class GroupedFp8Mixin:
             used = getattr(x, "_sg_rows", None)
         dy8, dy_inv = self._gq(ext, dy, True, used, self._gslot(ctx.layer, role, "dy"))
         w8, w_inv = self._expert_weight(ctx, ext, role, w)
-        dx = (torch.empty if used is not None else torch.zeros)(x.shape, dtype=torch.bfloat16, device=x.device)
+        dx = grouped_output(ext, x.shape, x, plan, used)
         ext.gemm_grouped(dy8, w8, dx, plan.offsets, 1, True, False, 1.0, dy_inv, w_inv, err)          # dy [R, N] . W[e] [N, K]
         if used is not None:
             dx._sg_rows = used

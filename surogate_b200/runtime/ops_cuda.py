@@ -403,6 +403,19 @@ class CudaOps(RefOps):
         return (total,)
 
 
+def grouped_output(ext, shape, like, plan, used):
+    """Output buffer of a grouped GEMM over rows.  Every row of a group (padding included) is written by the GEMM.  The rows behind the
+    last group are never read into a result: with a device row count in use (``used``, expert parallel) the buffer is only tagged with it
+    by the caller, otherwise those rows are zeroed."""
+    out = torch.empty(shape, dtype=torch.bfloat16, device=like.device)
+    if used is None:
+        if isinstance(plan, CudaMoEPlan) and out.dim() == 2 and out.shape[1] % 8 == 0:
+            ext.moe_zero_rows(out, plan.offsets)
+        else:
+            out.zero_()
+    return out
+
+
 class CudaMoEPlan:
     """Device-side routing plan: padded per-expert row ranges and the row each (token, k) copy landed on."""
 
@@ -482,7 +495,11 @@ def _moe_mixin():
         cursors = torch.empty(E, dtype=torch.int32, device=x.device)
         self.ext.moe_offsets(counts, offsets, cursors, cap, self.ext.error_flag_tensor())
         row_map = torch.empty(N * K, dtype=torch.int32, device=x.device)
-        xp = torch.zeros(cap, C, dtype=x.dtype, device=x.device)   # pad rows must be zero (they enter the wgrad contraction)
+        xp = torch.empty(cap, C, dtype=x.dtype, device=x.device)
+        if C % 8 == 0:
+            self.ext.moe_zero_rows(xp, offsets, counts)                # pad rows must be zero (they enter the wgrad contraction)
+        else:
+            xp.zero_()
         self.ext.moe_permute(x2, ti.reshape(N, K).contiguous(), offsets, cursors, row_map, xp, 0, E)
         return xp, CudaMoEPlan(row_map, offsets, counts, cap, N, K, E, tuple(x.shape))
 
@@ -505,9 +522,7 @@ def _moe_mixin():
                 r = ctx.lora.forward_grouped(ctx, op, x, r, plan)
             return (r,)
         used = getattr(x, "_sg_rows", None)
-        # every row of a group (padding included) is written by the GEMM; rows behind the last group are never read into a result,
-        # so a buffer sized for the worst case (expert parallel) is not cleared, only tagged with the row count in use
-        y = (torch.empty if used is not None else torch.zeros)(x.shape[0], w.shape[1], dtype=x.dtype, device=x.device)
+        y = grouped_output(self.ext, (x.shape[0], w.shape[1]), x, plan, used)
         self.ext.gemm_grouped(x, w, y, plan.offsets, 1, False, False, 1.0, None, None, self.ext.error_flag_tensor())
         if used is not None:
             y._sg_rows = used
@@ -535,7 +550,7 @@ def _moe_mixin():
         used = getattr(dy, "_sg_rows", None)
         if used is None:
             used = getattr(x, "_sg_rows", None)
-        dx = (torch.empty_like if used is not None else torch.zeros_like)(x)
+        dx = grouped_output(self.ext, x.shape, x, plan, used)
         self.ext.gemm_grouped(dy, w, dx, plan.offsets, 1, True, False, 1.0, None, None, err)     # dy [R,N] . W[g] [N,K]
         if used is not None:
             dx._sg_rows = used
@@ -562,7 +577,8 @@ def _moe_mixin():
         plan = plan.local or plan
         if not isinstance(plan, CudaMoEPlan):
             return RefOps.moe_unpermute_backward(self, ctx, op, dy, yp, tw, plan)
-        d_yp, d_tw = self.ext.moe_unpermute_bwd(dy.reshape(plan.num_tokens, -1).contiguous(), yp, tw.reshape(-1, plan.top_k).contiguous(), plan.row_map)
+        d_yp, d_tw = self.ext.moe_unpermute_bwd(dy.reshape(plan.num_tokens, -1).contiguous(), yp, tw.reshape(-1, plan.top_k).contiguous(), plan.row_map,
+                                                plan.offsets, plan.counts)
         return d_yp, d_tw.reshape(tw.shape)
 
     def ep_dispatch(self, ctx, op, xp, plan):

@@ -638,6 +638,30 @@ def test_moe_permute_grouped_gemm_unpermute(ext):
     _check_flag()
 
 
+@pytest.mark.parametrize("E,cap,C,pads", [(1, 128, 8, True), (8, 4096, 64, True), (128, 40000, 24, True), (8, 2048, 256, False), (4, 512, 16, True)])
+def test_moe_zero_rows(ext, E, cap, C, pads):
+    """Exactly the rows that no token owns are cleared: the padding of each group (with counts) and the tail; empty groups, full groups and a
+    buffer with no tail."""
+    g = torch.Generator().manual_seed(E + cap)
+    counts = torch.randint(0, 400, (E,), generator=g)
+    counts[0] = 128
+    if E > 2:
+        counts[2] = 0
+    if E == 4:
+        counts[:] = 128
+    padded = (counts + 127) // 128 * 128
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), padded.cumsum(0)])
+    cap = max(cap, int(offsets[-1])) if E != 4 else int(offsets[-1])
+    buf = torch.full((cap, C), 7.0, device=DEV, dtype=torch.bfloat16)
+    ext.moe_zero_rows(buf, offsets.int().to(DEV), counts.int().to(DEV) if pads else None)
+    want = torch.full((cap, C), 7.0)
+    want[int(offsets[-1]):] = 0
+    if pads:
+        for e in range(E):
+            want[int(offsets[e] + counts[e]):int(offsets[e + 1])] = 0
+    assert torch.equal(buf.float().cpu(), want)
+
+
 def test_embedding_rejects_out_of_range_token_ids():
     """An invalid token id must not read outside the table: the row is zero-filled and the error flag is raised."""
     from surogate_b200.ops import check_device_errors, ext
