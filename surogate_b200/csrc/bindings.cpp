@@ -7,6 +7,7 @@
 #include <cstdlib>
 
 #include "gemm_sm100.h"
+#include "step_kernels.h"
 #include "kernels.h"
 #include "ext_api.h"
 
@@ -267,8 +268,9 @@ std::vector<Tensor> qk_norm_rope_bwd(const Tensor& d_out, const Tensor& qkv_pre,
     const bool norm = qw.has_value() && qw->defined();
     Tensor dqw, dkw;
     if (norm) {
-        dqw = torch::zeros({D}, d_out.options().dtype(at::kFloat));
-        dkw = torch::zeros({D}, d_out.options().dtype(at::kFloat));
+        const Tensor both = torch::zeros({2, D}, d_out.options().dtype(at::kFloat));
+        dqw = both.select(0, 0);
+        dkw = both.select(0, 1);
     }
     g_launches += 1;
     sg::qk_norm_rope_bwd(d_out.data_ptr(), qkv_pre.data_ptr(), opt_ptr(qw), opt_ptr(kw), pos.data_ptr<int>(), dx.data_ptr(), opt_f32_mut(q_rstd),
@@ -412,6 +414,64 @@ Tensor sumsq(const Tensor& x) {
     return partial.sum();
 }
 
+// [sum of squares of all `dense`, sum of squares of all `experts`], fp32
+Tensor sumsq_groups(const std::vector<Tensor>& dense, const std::vector<Tensor>& experts, const Tensor& like) {
+    const c10::cuda::CUDAGuard guard(like.device());
+    const int nblocks = num_sms() * 2, n = static_cast<int>(dense.size() + experts.size());
+    Tensor out = torch::empty({2}, like.options().dtype(at::kFloat));
+    Tensor partial = torch::empty({static_cast<int64_t>(n) * nblocks}, out.options());
+    float* dst = n ? partial.data_ptr<float>() : nullptr;
+    for (const auto* group : {&dense, &experts})
+        for (const Tensor& x : *group) {
+            check_cuda(x, "x");
+            TORCH_CHECK(x.is_contiguous() && (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16), "sumsq: contiguous fp32/bf16");
+            sg::sumsq(x.data_ptr(), x.scalar_type() == at::kFloat, dst, nblocks, x.numel(), cur_stream());
+            dst += nblocks;
+        }
+    g_launches += n + 1;
+    sg::sum_partials(n ? partial.data_ptr<float>() : out.data_ptr<float>(), static_cast<int>(dense.size()) * nblocks, n * nblocks, out.data_ptr<float>(), cur_stream());
+    return out;
+}
+
+static float* scalar_f32(const Tensor& t, const char* what) {
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.numel() == 1, what, ": one CUDA float32");
+    return t.data_ptr<float>();
+}
+
+// [valid targets, 1 / max(valid, 1)]
+Tensor count_targets(const Tensor& targets, int64_t ignore) {
+    TORCH_CHECK(targets.is_cuda() && targets.scalar_type() == at::kInt && targets.is_contiguous(), "targets must be contiguous CUDA int32");
+    const c10::cuda::CUDAGuard guard(targets.device());
+    Tensor out = torch::empty({2}, targets.options().dtype(at::kFloat));
+    g_launches += 1;
+    sg::count_targets(targets.data_ptr<int>(), targets.numel(), static_cast<int>(ignore), out.data_ptr<float>(), cur_stream());
+    return out;
+}
+
+// Fills the hyper-parameter vector (clip factor from `total`, the squared gradient norm) and returns the norm.
+Tensor step_hyper(Tensor& hp, const Tensor& total, const std::vector<double>& host, double max_norm) {
+    TORCH_CHECK(hp.is_cuda() && hp.scalar_type() == at::kFloat && hp.is_contiguous() && hp.numel() >= 8 && host.size() == 7, "step_hyper: hp [8], seven host values");
+    const c10::cuda::CUDAGuard guard(hp.device());
+    Tensor norm = torch::empty({}, hp.options());
+    sg::StepHyper h;
+    for (int i = 0; i < 7; ++i) h.v[i] = static_cast<float>(host[i]);
+    h.max_norm = static_cast<float>(max_norm);
+    g_launches += 1;
+    sg::step_hyper(scalar_f32(total, "total"), h, hp.data_ptr<float>(), norm.data_ptr<float>(), cur_stream());
+    return norm;
+}
+
+// [mean loss + aux, norm, aux, device error flag]
+Tensor step_report(const Tensor& loss_sum, const Tensor& n_valid, const Tensor& aux, const Tensor& norm) {
+    const c10::cuda::CUDAGuard guard(loss_sum.device());
+    Tensor out = torch::empty({4}, loss_sum.options());
+    const int* flag = error_flag_ptr();
+    g_launches += 1;
+    sg::step_report(scalar_f32(loss_sum, "loss"), scalar_f32(n_valid, "n_valid"), scalar_f32(aux, "aux"), scalar_f32(norm, "norm"), flag, out.data_ptr<float>(),
+                    cur_stream());
+    return out;
+}
+
 void adamw_step(Tensor& p, const Tensor& g, Tensor& m, Tensor& v, const c10::optional<Tensor>& mask, const Tensor& hp) {
     check_cuda(p, "p");
     TORCH_CHECK(p.is_contiguous() && g.is_contiguous() && m.is_contiguous() && v.is_contiguous(), "adamw: contiguous tensors");
@@ -476,6 +536,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("dequantize_fp8", &dequantize_fp8);
     m.def("amax", &amax, pybind11::arg("x"), pybind11::arg("amax_out"), pybind11::arg("rows_limit") = c10::optional<Tensor>());
     m.def("sumsq", &sumsq);
+    m.def("sumsq_groups", &sumsq_groups);
+    m.def("count_targets", &count_targets);
+    m.def("step_hyper", &step_hyper);
+    m.def("step_report", &step_report);
     m.def("adamw_step", &adamw_step);
     m.def("adamw8_step", &adamw8_step);
     sg_register_extra(m);

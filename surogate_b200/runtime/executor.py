@@ -349,11 +349,11 @@ class Executor:
         tgt, acc = ctx.grad_target(out_name)
         if tgt is None:
             return
-        v = val.reshape(tgt.shape).to(tgt.dtype)
+        v = val.reshape(tgt.shape)
         if acc:
-            tgt.add_(v)
+            tgt.add_(v.to(tgt.dtype))
         else:
-            tgt.copy_(v)
+            tgt.copy_(v)      # converts as it copies
 
     # ------------------------------------------------------------------ block stack
     def _block_stack_forward(self, op: OpNode, env, ctx: ExecContext):

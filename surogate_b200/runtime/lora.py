@@ -322,6 +322,10 @@ class LoRAManager:
             self.comm.all_reduce(self.grad, "sum")
 
     def grad_sumsq(self) -> torch.Tensor:
+        if self.use_kernels:
+            from ..ops import ext
+
+            return ext().sumsq(self.grad)
         return self.grad.pow(2).sum()
 
     def optimizer_step(self, hp: torch.Tensor, hp_host) -> None:

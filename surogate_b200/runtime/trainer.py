@@ -364,10 +364,14 @@ class Trainer:
             doc_ids = None
             if bool((position_ids[:, 1:] <= position_ids[:, :-1]).any()) if isinstance(position_ids, np.ndarray) else False:
                 doc_ids = torch.cumsum((pos == 0).to(torch.int32), dim=1)  # packed documents: id increments at each reset
-        n_valid = (tgt != -100).sum().to(torch.float32)
-        if self.world > 1:
-            self.comm.all_reduce(n_valid, "sum")
-        loss_scale = (1.0 / n_valid.clamp_min(1.0)).reshape(1)
+        if self._native and self.world == 1 and tgt.numel() <= 65536:      # one block counts; larger batches keep the parallel reduction
+            count = self.backend.ext.count_targets(tgt.contiguous(), -100)
+            n_valid, loss_scale = count[0], count[1:]
+        else:
+            n_valid = (tgt != -100).sum().to(torch.float32)
+            if self.world > 1:
+                self.comm.all_reduce(n_valid, "sum")
+            loss_scale = (1.0 / n_valid.clamp_min(1.0)).reshape(1)
         if loss_scale_override is not None:
             loss_scale = torch.full((1,), float(loss_scale_override), dtype=torch.float32, device=self.device)
         if row_weights is not None:
@@ -498,26 +502,35 @@ class Trainer:
             total[1] = total[1] / N  # the auxiliary loss is a per-piece mean
         return ctx, total
 
+    @property
+    def _native(self) -> bool:
+        return self.device.type == "cuda" and self.backend.name == "cuda"
+
     def grad_norm(self) -> torch.Tensor:
-        """Global L2 norm of the (already reduced) gradients, as a device scalar.
+        """Global L2 norm of the (already reduced) gradients, as a device scalar."""
+        return self._grad_sumsq().sqrt()
+
+    def _grad_sumsq(self) -> torch.Tensor:
+        """Its square.
 
         Three kinds of terms, each counted exactly once: dense buckets (replicated after an all-reduce, or one shard per rank under
         ZeRO), expert buckets (one copy per rank of an expert group; with an expert-parallel x data-parallel mesh the same copy exists
         in every replica of the group) and the adapter buffer (already all-reduced, identical everywhere)."""
-        on_gpu = self.device.type == "cuda" and self.backend.name == "cuda"
-
         def sumsq(g):
-            return self.backend.ext.sumsq(g) if on_gpu else g.float().pow(2).sum()
+            return self.backend.ext.sumsq(g) if self._native else g.float().pow(2).sum()
 
         fused = self.store.fused_sumsq is not None and self.store.sumsq_valid and self.lora is None
-        parts = torch.zeros(2, dtype=torch.float32, device=self.device)   # [dense, experts]
+        groups = ([], [])                                                                  # dense, experts
         for b in self.store.trainable_buckets():
-            if b.grad_shard is None:
-                continue
-            if b.expert:
-                parts[1] += sumsq(b.grad_shard)
-            elif not fused:
-                parts[0] += sumsq(b.grad_shard)
+            if b.grad_shard is not None and (b.expert or not fused):
+                groups[1 if b.expert else 0].append(b.grad_shard)
+        if self._native:
+            parts = self.backend.ext.sumsq_groups(groups[0], groups[1], self._hp)
+        else:
+            parts = torch.zeros(2, dtype=torch.float32, device=self.device)
+            for i, gs in enumerate(groups):
+                for g in gs:
+                    parts[i] += sumsq(g)
         if fused:  # the reduce-scatter kernels already accumulated this rank's shard norms
             parts[0] += self.store.fused_sumsq.reshape(())
             if os.environ.get("SUROGATE_CHECK_FUSED_NORM") == "1":  # self-check: recompute from the reduced shards
@@ -535,7 +548,7 @@ class Trainer:
         if self.lora is not None:
             # the adapter gradient is already all-reduced (identical on every rank): it joins after the cross-rank sum
             total = total + self.lora.grad_sumsq()
-        return total.sqrt()
+        return total
 
     def drain_optimizer(self) -> None:
         """With ``async_optimizer``: wait for the update in flight and make its weights the ones the next step reads."""
@@ -553,13 +566,17 @@ class Trainer:
         self._steps_here = getattr(self, "_steps_here", 0) + 1
         t = self.step_index
         lr = cfg.learning_rate if lr is None else lr
-        norm = self.grad_norm() if norm is None else norm
-        clip = torch.clamp(cfg.max_grad_norm / (norm + 1e-6), max=1.0) if cfg.max_grad_norm and cfg.max_grad_norm > 0 else torch.ones_like(norm)
-        clip = torch.where(torch.isfinite(norm), clip, torch.zeros_like(clip))  # a non-finite norm skips the update: the optimizer kernels and CPU paths return early on a zero scale
         host = (lr, cfg.beta1, cfg.beta2, cfg.eps, cfg.weight_decay, 1 - cfg.beta1 ** t, 1 - cfg.beta2 ** t)
-        hp_cpu = torch.tensor(list(host) + [1.0], dtype=torch.float32)
-        self._hp.copy_(hp_cpu, non_blocking=True)
-        self._hp[7] = clip
+        if norm is None and self._native:
+            norm = self.backend.ext.step_hyper(self._hp, self._grad_sumsq(), list(host), float(cfg.max_grad_norm or 0.0))
+            clip = self._hp[7]
+        else:
+            norm = self.grad_norm() if norm is None else norm
+            clip = torch.clamp(cfg.max_grad_norm / (norm + 1e-6), max=1.0) if cfg.max_grad_norm and cfg.max_grad_norm > 0 else torch.ones_like(norm)
+            clip = torch.where(torch.isfinite(norm), clip, torch.zeros_like(clip))  # a non-finite norm skips the update: the optimizer kernels and CPU paths return early on a zero scale
+            hp_cpu = torch.tensor(list(host) + [1.0], dtype=torch.float32)
+            self._hp.copy_(hp_cpu, non_blocking=True)
+            self._hp[7] = clip
         fence = getattr(self.comm, "fence", None)
         if fence is not None:
             fence()  # every rank has finished reading master shards / gradient buckets of this step
@@ -593,15 +610,20 @@ class Trainer:
         if timer is not None:
             timer.mark("optimizer")
             self.last_time_breakdown = timer.totals()
-        loss = r["loss_sum"].clone()
+        loss = r["loss_sum"]
         if self.world > 1:
+            loss = loss.clone()
             self.comm.all_reduce(loss, "sum")
-        out = torch.stack([loss / r["n_valid"].clamp_min(1.0) + r["aux"], norm, r["aux"]]).to("cpu")  # the step's only D2H sync
-        self.d2h_bytes += out.numel() * 4
-        if self.device.type == "cuda" and self.backend.name == "cuda":
-            from ..ops import check_device_errors
+        if self._native:
+            out = self.backend.ext.step_report(loss, r["n_valid"], r["aux"], norm).to("cpu")  # the step's only D2H sync
+            self.d2h_bytes += out.numel() * 4
+            if float(out[3]) != 0:
+                from ..ops import check_device_errors
 
-            check_device_errors()
+                check_device_errors()
+        else:
+            out = torch.stack([loss / r["n_valid"].clamp_min(1.0) + r["aux"], norm, r["aux"]]).to("cpu")
+            self.d2h_bytes += out.numel() * 4
         return {"loss": float(out[0]), "norm": float(out[1]), "aux_loss": float(out[2])}
 
     # ------------------------------------------------------------------ call-compatible spellings of the reference's Python API

@@ -439,6 +439,31 @@ def test_dequantize_fp8(ext, shape, dt):
     assert out.shape == q.shape and torch.equal(out, (q.float() * scale).bfloat16())
 
 
+@pytest.mark.parametrize("n", [1, 31, 1024, 5000])
+def test_step_scalars(ext, n):
+    """Target count and loss scale, squared norms, clip factor (also without a limit and for a norm that is not finite) and the step's record."""
+    torch.manual_seed(n)
+    tgt = torch.randint(0, 50, (n,), device=DEV, dtype=torch.int32)
+    tgt[torch.rand(n, device=DEV) < 0.3] = -100
+    valid = int((tgt != -100).sum())
+    c = ext.count_targets(tgt, -100)
+    assert c[0].item() == valid and abs(c[1].item() - 1 / max(valid, 1)) < 1e-7
+    assert ext.count_targets(torch.full((n,), -100, device=DEV, dtype=torch.int32), -100).tolist() == [0.0, 1.0]
+    a, b, e = torch.randn(8 * n, device=DEV).bfloat16(), torch.randn(n, device=DEV), torch.randn(4096, device=DEV).bfloat16()
+    hp = torch.zeros(8, device=DEV)
+    sq = ext.sumsq_groups([a, b], [e], hp)
+    assert abs(sq[0].item() / (a.double().pow(2).sum() + b.double().pow(2).sum()).item() - 1) < 1e-5
+    assert abs(sq[1].item() / e.double().pow(2).sum().item() - 1) < 1e-5
+    assert ext.sumsq_groups([], [], hp).tolist() == [0.0, 0.0]
+    host = [1e-3, 0.9, 0.99, 1e-8, 0.1, 0.19, 0.02]
+    for total, limit, clip in [(16.0, 1.0, 1.0 / (4.0 + 1e-6)), (0.25, 1.0, 1.0), (16.0, 0.0, 1.0), (float("inf"), 1.0, 0.0), (float("nan"), 0.0, 0.0)]:
+        norm = ext.step_hyper(hp, torch.tensor(total, device=DEV), host, limit)
+        torch.testing.assert_close(hp.cpu(), torch.tensor(host + [clip]))
+        assert norm.shape == () and (norm.item() == total ** 0.5 or total != total)
+    out = ext.step_report(torch.tensor(6.0, device=DEV), c[0], torch.tensor(0.5, device=DEV), torch.tensor(2.0, device=DEV))
+    torch.testing.assert_close(out.cpu(), torch.tensor([6.0 / max(valid, 1) + 0.5, 2.0, 0.5, 0.0]))
+
+
 def test_adamw_kernels(ext):
     n = 100000 - 100000 % 32
     p = torch.randn(n, device=DEV)
