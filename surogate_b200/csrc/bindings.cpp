@@ -363,6 +363,26 @@ Tensor cross_entropy_fwd_bwd(Tensor& logits, const Tensor& targets, const c10::o
     return loss;
 }
 
+// Loss per row and d(logits) as E5M2 of gradient * q_scale, [rows, V]; the logits are left alone.
+std::vector<Tensor> cross_entropy_fwd_bwd_fp8(const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& scale, double scale_host,
+                                              const Tensor& q_scale) {
+    check_cuda(logits, "logits");
+    TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && logits.dim() == 2 && logits.stride(1) == 1, "logits must be 2-D bf16 with contiguous rows");
+    TORCH_CHECK(targets.is_cuda() && targets.scalar_type() == at::kInt && targets.is_contiguous(), "targets must be contiguous CUDA int32");
+    const int rows = static_cast<int>(logits.size(0)), V = static_cast<int>(logits.size(1)), ld = static_cast<int>(logits.stride(0));
+    TORCH_CHECK(V % 8 == 0 && ld % 8 == 0, "cross_entropy: V and row stride must be multiples of 8");
+    TORCH_CHECK(targets.numel() == rows, "one target per row");
+    TORCH_CHECK(q_scale.is_cuda() && q_scale.scalar_type() == at::kFloat && q_scale.numel() >= 1, "q_scale: one CUDA float32");
+    const c10::cuda::CUDAGuard guard(logits.device());
+    Tensor loss = torch::empty({rows}, logits.options().dtype(at::kFloat));
+    Tensor d8 = torch::empty({rows, V}, logits.options().dtype(at::kFloat8_e5m2));
+    if (rows == 0) return {loss, d8};
+    g_launches += 1;
+    sg::cross_entropy_fwd_bwd_fp8(logits.data_ptr(), d8.data_ptr(), q_scale.data_ptr<float>(), targets.data_ptr<int>(), loss.data_ptr<float>(), opt_f32(scale),
+                                  static_cast<float>(scale_host), rows, V, ld, cur_stream());
+    return {loss, d8};
+}
+
 Tensor quantize_fp8(const Tensor& x, const c10::optional<Tensor>& scale, const c10::optional<Tensor>& amax_out, bool e5m2,
                     const c10::optional<Tensor>& rows_limit, const c10::optional<Tensor>& out) {
     check_bf16(x, "x");
@@ -531,6 +551,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("cross_entropy_fwd_bwd", &cross_entropy_fwd_bwd, py::arg("logits"), py::arg("targets"), py::arg("scale"), py::arg("scale_host"),
           py::arg("write_grad"), py::arg("row_weight") = py::none(), py::arg("kd_idx") = py::none(), py::arg("kd_logp") = py::none(),
           py::arg("kd_weight") = 0.0, py::arg("kd_loss_out") = py::none());
+    m.def("cross_entropy_fwd_bwd_fp8", &cross_entropy_fwd_bwd_fp8, py::arg("logits"), py::arg("targets"), py::arg("scale"), py::arg("scale_host"), py::arg("q_scale"));
     m.def("quantize_fp8", &quantize_fp8, pybind11::arg("x"), pybind11::arg("scale"), pybind11::arg("amax_out"), pybind11::arg("e5m2"),
           pybind11::arg("rows_limit") = c10::optional<Tensor>(), pybind11::arg("out") = c10::optional<Tensor>());
     m.def("dequantize_fp8", &dequantize_fp8);

@@ -29,6 +29,8 @@ void embedding_bwd(const int* tokens, const void* d_out, void* d_table, int grad
 void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V,
                           cudaStream_t s);
 void dequantize_fp8(const void* q, const float* scale, void* out, size_t n, int e5m2, int num_sms, cudaStream_t s);
+void cross_entropy_fwd_bwd_fp8(const void* logits, void* d8, const float* q_scale, const int* targets, float* loss, const float* scale_ptr, float scale_host, int rows,
+                               int V, int ld, cudaStream_t s);
 void cross_entropy_fwd_bwd(void* logits, const int* targets, float* loss, const float* scale_ptr, float scale_host, int rows, int V, int ld,
                            int write_grad, const float* row_weight, const int* kd_idx, const float* kd_logp, int kd_k, float kd_weight, float* kd_loss,
                            cudaStream_t s);

@@ -377,16 +377,17 @@ class CudaOps(RefOps):
                 gemm(x8[s:e], w8, lg, scale_a=x_inv, scale_b=w_inv)
             else:
                 gemm(x2[s:e], w, lg)
-            losses[s:e] = self.ext.cross_entropy_fwd_bwd(lg, t[s:e], scale_t, scale_h, train, rw[s:e] if rw is not None else None,
-                                                         kd_idx[s:e] if kd else None, kd_logp[s:e] if kd else None, float(kd["weight"]) if kd else 0.0,
-                                                         kd_losses[s:e] if kd else None)
-            if train and fp8:
-                d8 = self.ext.quantize_fp8(lg, d_scale, None, True)
+            if train and fp8:   # the E5M2 gradient comes straight out of the loss kernel
+                losses[s:e], d8 = self.ext.cross_entropy_fwd_bwd_fp8(lg, t[s:e], scale_t, scale_h, d_scale)
                 gemm(d8, w8, dx[s:e], a_mn=False, b_mn=True, scale_a=d_inv, scale_b=w_inv)
                 if tgt is not None:
                     gemm(d8, x8[s:e], tgt, a_mn=True, b_mn=True, accumulate=acc, scale_a=d_inv, scale_b=x_inv)
                     acc = True
-            elif train:
+                continue
+            losses[s:e] = self.ext.cross_entropy_fwd_bwd(lg, t[s:e], scale_t, scale_h, train, rw[s:e] if rw is not None else None,
+                                                         kd_idx[s:e] if kd else None, kd_logp[s:e] if kd else None, float(kd["weight"]) if kd else 0.0,
+                                                         kd_losses[s:e] if kd else None)
+            if train:
                 gemm(lg, w, dx[s:e], a_mn=False, b_mn=True)
                 if tgt is not None:
                     gemm(lg, x2[s:e], tgt, a_mn=True, b_mn=True, accumulate=acc)

@@ -286,6 +286,29 @@ def test_swiglu_row_counts(ext, rows, M):
     assert torch.equal(half[:rows // 2], y[:rows // 2])
 
 
+@pytest.mark.parametrize("V", [8, 4096, 8200, 32000, 151936])
+def test_cross_entropy_fp8_gradient(ext, V):
+    """The E5M2 gradient bit for bit against quantising the bf16 one, the same losses, untouched logits; rows with -inf logits and ignored
+    rows, and a row stride."""
+    torch.manual_seed(V)
+    rows = 6
+    wide = (3 * torch.randn(rows, V + 16, device=DEV)).bfloat16()
+    logits = wide[:, 8:8 + V] if V % 16 else wide[:, :V]
+    logits[1, : V // 2] = float("-inf")
+    logits[2] = 0
+    tgt = torch.randint(0, V, (rows,), device=DEV, dtype=torch.int32)
+    tgt[1] = V - 1
+    tgt[4] = -100
+    before = logits.clone()
+    ref_loss = torch.nn.functional.cross_entropy(logits.float(), tgt.long(), ignore_index=-100, reduction="none")
+    scale, q_scale = torch.tensor([0.5], device=DEV), torch.tensor([57344.0 * 0.5 / 0.25], device=DEV)
+    loss8, d8 = ext.cross_entropy_fwd_bwd_fp8(logits, tgt, scale, 0.5, q_scale)
+    assert torch.equal(logits, before)
+    loss = ext.cross_entropy_fwd_bwd(logits, tgt, scale, 0.5, True)
+    assert torch.allclose(loss, ref_loss, rtol=1e-4, atol=1e-4) and torch.equal(loss8, loss)
+    assert torch.equal(d8.view(torch.uint8), ext.quantize_fp8(logits.contiguous(), q_scale, None, True).view(torch.uint8)) and not logits[4].any()
+
+
 @pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
 @pytest.mark.parametrize("e5m2", [False, True])
 def test_quantize_fp8_counts(ext, n, e5m2):
