@@ -280,6 +280,20 @@ std::vector<Tensor> qk_norm_rope_bwd(const Tensor& d_out, const Tensor& qkv_pre,
     return {dx, dqw, dkw};
 }
 
+// t.zero_() for a contiguous tensor
+void zero_fill(Tensor& t) {
+    check_cuda(t, "t");
+    const size_t bytes = t.numel() * t.element_size();
+    if (!t.is_contiguous() || bytes % 16 != 0 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0) {
+        t.zero_();
+        return;
+    }
+    if (bytes == 0) return;
+    const c10::cuda::CUDAGuard guard(t.device());
+    g_launches += 1;
+    sg::zero_fill(t.data_ptr(), bytes, num_sms(), cur_stream());
+}
+
 Tensor embedding_fwd(const Tensor& tokens, const Tensor& table) {
     check_bf16(table, "table");
     TORCH_CHECK(tokens.is_cuda() && tokens.scalar_type() == at::kInt && tokens.is_contiguous(), "tokens must be contiguous CUDA int32");
@@ -303,6 +317,18 @@ void embedding_bwd(const Tensor& tokens, const Tensor& d_out, Tensor& d_table, b
         TORCH_CHECK(d_table.is_cuda() && d_table.is_contiguous() && (d_table.scalar_type() == at::kFloat || d_table.scalar_type() == at::kBFloat16) &&
                         d_table.size(1) % 2 == 0,
                     "d_table: contiguous fp32 / bf16 [V, C]");
+        // rows of whole 16-byte vectors go through the kernel below; other widths and misaligned views through padded copies
+        if (d_table.size(1) % 8 != 0 || (reinterpret_cast<uintptr_t>(d_table.data_ptr()) & 15) != 0 || (reinterpret_cast<uintptr_t>(d_out.data_ptr()) & 15) != 0) {
+            const c10::cuda::CUDAGuard guard2(d_out.device());
+            const int64_t C = d_table.size(1), Cp = (C + 7) / 8 * 8;
+            Tensor padded = torch::zeros({d_table.size(0), Cp}, d_table.options());
+            padded.narrow(1, 0, C).copy_(d_table);
+            Tensor rows = torch::zeros({d_out.numel() / C, Cp}, d_out.options());
+            rows.narrow(1, 0, C).copy_(d_out.reshape({-1, C}));
+            embedding_bwd(tokens, rows, padded, true);
+            d_table.copy_(padded.narrow(1, 0, C));
+            return;
+        }
         const c10::cuda::CUDAGuard guard(d_out.device());
         auto sorted = tokens.reshape({-1}).sort(/*stable=*/true, /*dim=*/0, /*descending=*/false);
         Tensor ids = std::get<0>(sorted).contiguous(), order = std::get<1>(sorted).contiguous();
@@ -547,6 +573,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("k_rstd"), py::arg("position_ids"), py::arg("num_q_heads"), py::arg("num_kv_heads"), py::arg("head_dim"), py::arg("eps"), py::arg("theta"),
           py::arg("sec_h") = 0, py::arg("sec_w") = 0);
     m.def("embedding_fwd", &embedding_fwd);
+    m.def("zero_fill", &zero_fill);
     m.def("embedding_bwd", &embedding_bwd, py::arg("tokens"), py::arg("d_out"), py::arg("d_table"), py::arg("deterministic") = true);
     m.def("cross_entropy_fwd_bwd", &cross_entropy_fwd_bwd, py::arg("logits"), py::arg("targets"), py::arg("scale"), py::arg("scale_host"),
           py::arg("write_grad"), py::arg("row_weight") = py::none(), py::arg("kd_idx") = py::none(), py::arg("kd_logp") = py::none(),

@@ -103,7 +103,7 @@ class CudaOps(RefOps):
         if tgt is None:
             return (None,)
         if not acc:
-            tgt.zero_()
+            self.ext.zero_fill(tgt)
         self.ext.embedding_bwd(token_ids.contiguous(), d_x.contiguous(), tgt)
         return (None,)
 

@@ -309,6 +309,30 @@ def test_cross_entropy_fp8_gradient(ext, V):
     assert torch.equal(d8.view(torch.uint8), ext.quantize_fp8(logits.contiguous(), q_scale, None, True).view(torch.uint8)) and not logits[4].any()
 
 
+@pytest.mark.parametrize("n,V,C", [(1, 4, 8), (7, 3, 512), (64, 2, 520), (1000, 50, 1032), (300, 7, 6), (257, 1, 24)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_embedding_gradient_runs(ext, n, V, C, dt):
+    """Runs of equal ids of one, around the eight rows in flight, and hundreds; column counts around a CTA's 512 and one that is not a
+    multiple of 8; ids outside the table; accumulation into a table, twice the same bits."""
+    torch.manual_seed(n + C)
+    ids = torch.randint(0, V + 1, (n,), device=DEV, dtype=torch.int32)        # V itself is outside: skipped
+    if V == 1:
+        ids[:] = 0
+    d = torch.randn(n, C, device=DEV).bfloat16()
+    start = torch.randn(V, C, device=DEV).to(dt)
+    a, b = start.clone(), start.clone()
+    ext.embedding_bwd(ids, d, a)
+    ext.embedding_bwd(ids, d, b)
+    keep = ids < V
+    want = start.double().index_add(0, ids[keep].long(), d[keep].double())
+    assert torch.equal(a, b)
+    scale = start.double().abs().index_add(0, ids[keep].long(), d[keep].double().abs())
+    assert ((a.double() - want).abs() <= (2.0 ** -8 if dt == torch.bfloat16 else 0.0) * want.abs() + n * 2.0 ** -24 * scale).all()
+    t = torch.randn(V, C, device=DEV).to(dt)
+    ext.zero_fill(t)
+    assert not t.any()
+
+
 @pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
 @pytest.mark.parametrize("e5m2", [False, True])
 def test_quantize_fp8_counts(ext, n, e5m2):
