@@ -2,12 +2,19 @@
 from __future__ import annotations
 
 
+_EXT = None
+
+
 def ext():
-    """The compiled extension module.  Raises with a clear message when it cannot be loaded."""
+    """The compiled extension module (loaded once per process).  Raises with a clear message when it cannot be loaded."""
+    global _EXT
+    if _EXT is not None:
+        return _EXT
     from . import _build
 
     try:
-        return _build.load()
+        _EXT = _build.load()
+        return _EXT
     except Exception as e:  # noqa: BLE001
         raise RuntimeError(
             "surogate_b200 CUDA extension (sm_100a) is not available: build it with "

@@ -316,6 +316,11 @@ class Executor:
         program = self._programs.get(key)
         if program is None:   # bound methods, input classes and free lists are resolved once per (graph, op range, keep set)
             program = self._programs[key] = (bake_program(g, self.backend, set(keep), ops), ops)   # holding ``ops`` keeps its id unique
+        opt = self.options
+        if self.timer is None and self.op_profile is None and opt.dump_tensors is None and not opt.check_finite:
+            self._run_program(program[0], env, ctx, get_param)
+            ctx.graph = prev_graph
+            return
         for baked in program[0]:
             op = baked.op
             if self.timer is not None and op.kind == "fused_lm_head_loss":
@@ -344,6 +349,29 @@ class Executor:
             for n in baked.frees:
                 env.pop(n, None)
         ctx.graph = prev_graph
+
+    def _run_program(self, program, env: Dict[str, Any], ctx: ExecContext, get_param) -> None:
+        """The loop of ``run_graph`` without its instrumentation (timer, op profile, tensor dumps, finite checks)."""
+        prefix = f"blocks.{ctx.layer}." if ctx.layer is not None else ""
+        env_get, env_pop = env.get, env.pop
+        for baked in program:
+            op = baked.op
+            if baked.fn is not None:
+                outs = baked.fn(ctx, op, *[env_get(n) if c == 2 else (get_param(prefix + n) if c == 1 else None) for c, n in baked.sources])
+            elif op.kind == "block_stack":
+                outs = self._block_stack_forward(op, env, ctx)
+            else:
+                outs = self._block_stack_backward(op, env, ctx)
+            for name, val in zip(op.outputs, outs):
+                if name is None:
+                    continue
+                if name.startswith(GRAD_PREFIX):
+                    if val is not None:
+                        self._accumulate_grad(ctx, name, val)
+                else:
+                    env[name] = val
+            for n in baked.frees:
+                env_pop(n, None)
 
     def _accumulate_grad(self, ctx: ExecContext, out_name: str, val: torch.Tensor) -> None:
         tgt, acc = ctx.grad_target(out_name)

@@ -112,6 +112,16 @@ class _HostGatherWork:
         self.keep = None
 
 
+def _slot_view(flat: torch.Tensor, s) -> torch.Tensor:
+    """``flat[s.offset : s.offset + s.numel].view(s.shape)`` of a one-dimensional contiguous buffer, in one tensor operation: parameters are
+    looked up for every op of every layer."""
+    strides, n = [], 1
+    for d in reversed(s.shape):
+        strides.append(n)
+        n *= d
+    return flat.as_strided(s.shape, strides[::-1], flat.storage_offset() + s.offset)
+
+
 class ParamStore:
     def __init__(self, cm: CompiledModel, *, device, param_dtype=torch.float32, grad_dtype=None, master_dtype=None,
                  comm=None, zero_level: int = 0, keep_gathered: bool = True, frozen: Optional[Callable[[str], bool]] = None,
@@ -661,7 +671,7 @@ class ParamStore:
         b, s = self.where[name]
         if b.work is None or b.gather_work is not None or getattr(b, "_needs_post", False):
             self._ensure_gathered(b)
-        return b.work[s.offset:s.offset + s.numel].view(s.shape)
+        return _slot_view(b.work, s)
 
     # ------------------------------------------------------------------ gradients
     def begin_step(self) -> None:
@@ -691,7 +701,7 @@ class ParamStore:
             b.grad = torch.zeros(b.numel, dtype=self.grad_dtype, device=self.device)
         acc = name in b.written
         b.written.add(name)
-        return b.grad[s.offset:s.offset + s.numel].view(s.shape), acc
+        return _slot_view(b.grad, s), acc
 
     def _reduce_bucket(self, b: Bucket, zero_unwritten: bool = True) -> None:
         """Start the (async) gradient reduction of one bucket; called as soon as its backward is complete.
