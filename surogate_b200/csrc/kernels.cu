@@ -1215,8 +1215,7 @@ void adamw_8bit(void* p, int p_fp32, const void* g, int g_fp32, void* m8, void* 
 #define SG_A8(PT, GT, BM)                                                                                                                       \
     do {                                                                                                                                        \
         constexpr int smem = ADAM8_STAGES * adam8_slot_bytes<PT, GT>();                                                                           \
-        static const cudaError_t attr = cudaFuncSetAttribute(adamw_8bit_kernel<PT, GT, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);    \
-        (void)attr;                                                                                                                               \
+        cudaFuncSetAttribute(adamw_8bit_kernel<PT, GT, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   /* of the current device */        \
         const int grid = grid_for(n / 8, ADAM8_THREADS, num_sms, smem > 72 * 1024 ? 2 : 3);   /* the resident CTAs, each with a full ring */      \
         adamw_8bit_kernel<PT, GT, BM><<<grid, ADAM8_THREADS, smem, s>>>((PT*)p, (const GT*)g, (int8_t*)m8, (uint8_t*)v8, (__half*)ms, (__half*)vs, mask, hp, n); \
     } while (0)
