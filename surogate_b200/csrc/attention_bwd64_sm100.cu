@@ -10,8 +10,9 @@
 // Two groups of four softmax warps take alternate items.  Each group has its own pair of score accumulators (X, Y) in TMEM, reads them,
 // and writes P and dS as bf16 over them, from where the accumulating MMAs take their A operand: no copy in shared memory, no proxy
 // fence, and the room this leaves holds the fourth ring stage.  The MMA warp issues, per item, the accumulation of item i and then the
-// scores of item i + 2 into the same TMEM columns; MMAs of one thread execute in order, so the scores cannot overtake the reads of P and
-// dS.  While one group computes, the other's MMAs run.  Bound by the tensor pipe: a score MMA with 64 columns re-reads its resident operand
+// scores of item i + 2 into the same TMEM columns.  Only MMAs of the same accumulator and shape are ordered among themselves, so the scores
+// wait for a commit of the MMA that reads P (or dS) there: X(i + 2) for dV's, while dK's runs, and Y(i + 2) for dK's (dQ's), while X(i + 2)
+// runs, so that the tensor pipe has work during both waits.  While one group computes, the other's MMAs run.  Bound by the tensor pipe: a score MMA with 64 columns re-reads its resident operand
 // from shared memory at the full 128 bytes per cycle, which makes an item 1280 (dK/dV) or 1024 (dQ) cycles; measured 1530 and 1235, where
 // one set of eight warps that took one item at a time and paid each wait, TMEM read and fence in full needed 2155 for dK/dV.
 // Both passes on B200: 2 x 4096 x 32/8 heads 1313 -> 996 us, 1 x 8192 x 40/8 2912 -> 2222 us, 8 x 2048 x 16/8 705 -> 570 us.
@@ -100,8 +101,9 @@ constexpr int RING = 4;
 constexpr int OFF_R2 = T128, OFF_RING = 2 * T128, STAGE = 2 * T64, OFF_BAR = OFF_RING + RING * STAGE, OFF_VEC = OFF_BAR + 256;
 constexpr int VEC = 3 * 64 * 4;
 constexpr int SMEM = OFF_VEC + RING * VEC;
-// barriers: 0 res_full | 1-4 ring_full | 5-8 ring_empty | 9,10 xy_full | 11,12 pds_full | 13 done
-constexpr int B_RES = 0, B_RFULL = 1, B_REMPTY = B_RFULL + RING, B_XY = B_REMPTY + RING, B_PDS = B_XY + 2, B_DONE = B_PDS + 2;
+// barriers: 0 res_full | 1-4 ring_full | 5-8 ring_empty | 9,10 xy_full | 11,12 pds_full | 13 x_free | 14 y_free | 15 done
+constexpr int B_RES = 0, B_RFULL = 1, B_REMPTY = B_RFULL + RING, B_XY = B_REMPTY + RING, B_PDS = B_XY + 2, B_XFREE = B_PDS + 2, B_YFREE = B_XFREE + 1,
+              B_DONE = B_YFREE + 1;
 
 template <bool IS_DQ, bool HAS_LO>
 __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_constant__ CUtensorMap tm_qkv128, const __grid_constant__ CUtensorMap tm_qkv64,
@@ -190,7 +192,16 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
                 if (!mbar_wait(bar(B_RFULL + i % RING), (i / RING) & 1, abort_flag)) return false;
                 tc_fence_after();
                 const uint32_t c1 = s_ring + (i % RING) * STAGE, c2 = c1 + T64;
+                // item i - 2 left P and dS in these columns; in the dQ pass X holds no operand, only scores that have been read
+                if (!IS_DQ && i >= 2) {
+                    if (!mbar_wait(bar(B_XFREE), i & 1, abort_flag)) return false;
+                    tc_fence_after();
+                }
                 mma_128x64_kk(t_x[i & 1], s_r1, c1, idesc_s);     // S^T = K Q^T      |  S  = Q K^T
+                if (i >= 2) {
+                    if (!mbar_wait(bar(B_YFREE), i & 1, abort_flag)) return false;
+                    tc_fence_after();
+                }
                 mma_128x64_kk(t_y[i & 1], s_r2, c2, idesc_s);     // dP^T = V dO^T    |  dP = dO V^T
                 tc_commit(bar(B_XY + (i & 1)));
                 return true;
@@ -201,8 +212,12 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
                 if (!mbar_wait(bar(B_PDS + (i & 1)), (i >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t c1 = s_ring + (i % RING) * STAGE, c2 = c1 + T64;
-                if (!IS_DQ) mma_acc_k64(t_a2, t_x[i & 1], c2, idesc_acc, i > 0);     // dV += P^T dO
+                if (!IS_DQ) {
+                    mma_acc_k64(t_a2, t_x[i & 1], c2, idesc_acc, i > 0);             // dV += P^T dO
+                    tc_commit(bar(B_XFREE));
+                }
                 mma_acc_k64(t_a1, t_y[i & 1], c1, idesc_acc, i > 0);                 // dK += dS^T Q   |  dQ += dS K
+                tc_commit(bar(B_YFREE));
                 tc_commit(bar(B_REMPTY + i % RING));
                 if (i + 2 < n_items) ok = issue_xy(i + 2);                            // over P and dS of item i, behind their last reads
             }

@@ -135,6 +135,31 @@ def test_flash_attention_backward_item_counts(B, T, Hq, Hkv, window):
     _check_bwd(qkv, Hq, Hkv, _packed_lo(B, T, window, False) if window else None)
 
 
+@pytest.mark.parametrize("B,T,Hq,Hkv,window", [(1, 2048, 16, 2, 0), (2, 1024, 8, 8, 0), (1, 2048, 8, 2, 500)])
+def test_flash_attention_backward_repeats_its_bits(B, T, Hq, Hkv, window):
+    """The scores of an item are written over P and dS of the item two before it; nothing may depend on when the MMAs that read those
+    finish.  Long rows of items, beside other work and alone: always the same bits."""
+    from surogate_b200.ops import check_device_errors, ext
+
+    e = ext()
+    torch.manual_seed(T + Hq)
+    qkv = torch.randn(B, T, (Hq + 2 * Hkv) * D, device=DEV).bfloat16()
+    lo, qend = _packed_lo(B, T, window, False) if window else (None, None)
+    out, lse = e.flash_attn_fwd(qkv, Hq, Hkv, D ** -0.5, lo)
+    d_out = torch.randn_like(out)
+    first = e.flash_attn_bwd(d_out, qkv, out, lse, Hq, Hkv, D ** -0.5, lo, qend)
+    a = torch.randn(2048, 2048, device=DEV).bfloat16()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for i in range(20):
+        if i % 2:
+            with torch.cuda.stream(side):
+                a @ a
+        assert torch.equal(e.flash_attn_bwd(d_out, qkv, out, lse, Hq, Hkv, D ** -0.5, lo, qend), first)
+    torch.cuda.synchronize()
+    check_device_errors()
+
+
 def test_packed_batch_trains_like_the_masked_fp32_path():
     """One packed batch (position ids reset inside the rows) and one sliding-window model through the trainer on the CUDA backend:
     loss and gradient norm equal the PyTorch backend, whose attention applies the explicit document / window mask."""
