@@ -458,7 +458,11 @@ Tensor flash_attn_bwd(const Tensor& d_out, const Tensor& qkv, const Tensor& out,
     TORCH_CHECK(d_out.is_cuda() && d_out.scalar_type() == at::kBFloat16 && d_out.is_contiguous() && out.is_contiguous() && qkv.is_contiguous(), "bf16 contiguous");
     TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous(), "lse: fp32 contiguous");
     const int B = static_cast<int>(qkv.size(0)), T = static_cast<int>(qkv.size(1));
+    TORCH_CHECK(((reinterpret_cast<uintptr_t>(qkv.data_ptr()) | reinterpret_cast<uintptr_t>(d_out.data_ptr())) & 15) == 0,
+                "flash_attn_bwd: qkv and d_out must be 16-byte aligned");      // TMA, and vector loads of the row statistics
     const c10::cuda::CUDAGuard guard(qkv.device());
+    const bool out_aligned = (reinterpret_cast<uintptr_t>(out.data_ptr()) & 15) == 0;
+    const Tensor o = out_aligned ? out : out.clone();
     const int* lo_p = lo_ptr(lo, qkv);
     Tensor lo_copy;
     if (lo_p && (reinterpret_cast<uintptr_t>(lo_p) & 15) != 0) {   // the kernel copies 16 bytes at a time
@@ -475,7 +479,7 @@ Tensor flash_attn_bwd(const Tensor& d_out, const Tensor& qkv, const Tensor& out,
     Tensor d_qkv = torch::empty_like(qkv);
     Tensor stats = torch::empty({2 * lse.numel()}, lse.options());
     sg_count_launch(3);
-    const char* err = sg::flash_attn_bwd_sm100(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), stats.data_ptr<float>(),
+    const char* err = sg::flash_attn_bwd_sm100(qkv.data_ptr(), o.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), stats.data_ptr<float>(),
                                                d_qkv.data_ptr(), B, T, static_cast<int>(Hq), static_cast<int>(Hkv), static_cast<float>(scale),
                                                sg_error_flag(), sms(), cur_stream(), lo_p, qend_p);
     TORCH_CHECK(err == nullptr, err ? err : "");

@@ -160,6 +160,32 @@ def test_flash_attention_backward_repeats_its_bits(B, T, Hq, Hkv, window):
     check_device_errors()
 
 
+@pytest.mark.parametrize("shift", [4, 1])
+def test_flash_attention_backward_takes_a_misaligned_output(shift):
+    """The saved output may be a view that starts off a 16-byte boundary (elements of 2 bytes); d_out and qkv, which TMA reads, may not."""
+    from surogate_b200.ops import check_device_errors, ext
+
+    e = ext()
+    torch.manual_seed(shift)
+    Hq, Hkv = 4, 2
+    qkv = torch.randn(1, 256, (Hq + 2 * Hkv) * D, device=DEV).bfloat16()
+    out, lse = e.flash_attn_fwd(qkv, Hq, Hkv, D ** -0.5, None)
+    d_out = torch.randn_like(out)
+
+    def shifted(t):
+        v = torch.empty(t.numel() + 8, device=DEV, dtype=t.dtype)[shift:shift + t.numel()].view(t.shape)
+        return v.copy_(t)
+
+    want = e.flash_attn_bwd(d_out, qkv, out, lse, Hq, Hkv, D ** -0.5, None, None)
+    assert torch.equal(e.flash_attn_bwd(d_out, qkv, shifted(out), lse, Hq, Hkv, D ** -0.5, None, None), want)
+    with pytest.raises(RuntimeError):
+        e.flash_attn_bwd(shifted(d_out), qkv, out, lse, Hq, Hkv, D ** -0.5, None, None)
+    with pytest.raises(RuntimeError):
+        e.flash_attn_bwd(d_out, shifted(qkv), out, lse, Hq, Hkv, D ** -0.5, None, None)
+    torch.cuda.synchronize()
+    check_device_errors()
+
+
 def test_packed_batch_trains_like_the_masked_fp32_path():
     """One packed batch (position ids reset inside the rows) and one sliding-window model through the trainer on the CUDA backend:
     loss and gradient norm equal the PyTorch backend, whose attention applies the explicit document / window mask."""
