@@ -317,25 +317,15 @@ void embedding_bwd(const Tensor& tokens, const Tensor& d_out, Tensor& d_table, b
         TORCH_CHECK(d_table.is_cuda() && d_table.is_contiguous() && (d_table.scalar_type() == at::kFloat || d_table.scalar_type() == at::kBFloat16) &&
                         d_table.size(1) % 2 == 0,
                     "d_table: contiguous fp32 / bf16 [V, C]");
-        // rows of whole 16-byte vectors go through the kernel below; other widths and misaligned views through padded copies
-        if (d_table.size(1) % 8 != 0 || (reinterpret_cast<uintptr_t>(d_table.data_ptr()) & 15) != 0 || (reinterpret_cast<uintptr_t>(d_out.data_ptr()) & 15) != 0) {
-            const c10::cuda::CUDAGuard guard2(d_out.device());
-            const int64_t C = d_table.size(1), Cp = (C + 7) / 8 * 8;
-            Tensor padded = torch::zeros({d_table.size(0), Cp}, d_table.options());
-            padded.narrow(1, 0, C).copy_(d_table);
-            Tensor rows = torch::zeros({d_out.numel() / C, Cp}, d_out.options());
-            rows.narrow(1, 0, C).copy_(d_out.reshape({-1, C}));
-            embedding_bwd(tokens, rows, padded, true);
-            d_table.copy_(padded.narrow(1, 0, C));
-            return;
-        }
+        const uintptr_t bases = reinterpret_cast<uintptr_t>(d_table.data_ptr()) | reinterpret_cast<uintptr_t>(d_out.data_ptr());
+        const int vec = d_table.size(1) % 8 == 0 && bases % 16 == 0 ? 8 : (bases % 4 == 0 ? 2 : 1);
         const c10::cuda::CUDAGuard guard(d_out.device());
         auto sorted = tokens.reshape({-1}).sort(/*stable=*/true, /*dim=*/0, /*descending=*/false);
         Tensor ids = std::get<0>(sorted).contiguous(), order = std::get<1>(sorted).contiguous();
         g_launches += 1;
         sg::embedding_bwd_sorted(ids.data_ptr<int>(), reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), d_out.data_ptr(), d_table.data_ptr(),
                                  d_table.scalar_type() == at::kFloat, static_cast<int>(ids.numel()), static_cast<int>(d_table.size(1)),
-                                 static_cast<int>(d_table.size(0)), cur_stream());
+                                 static_cast<int>(d_table.size(0)), vec, cur_stream());
         return;
     }
     TORCH_CHECK(d_table.is_cuda() && d_table.is_contiguous(), "d_table must be contiguous CUDA");

@@ -581,16 +581,22 @@ template <typename G> __global__ void embedding_bwd_kernel(const int* __restrict
 // The longest run is the critical path (text repeats its frequent tokens hundreds of times per batch): EMB_AHEAD rows are requested before
 // the first is added, and the columns are spread over CTAs.  8192 rows of 4096, longest run 160, on B200: 577 -> 166 us with the sort
 // (about 100 us of it).
-constexpr int EMB_THREADS = 64, EMB_COLS = EMB_THREADS * 8, EMB_AHEAD = 8;
-template <typename G>
-__global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_kernel(const int* __restrict__ sorted_ids, const long long* __restrict__ order,
-                                                                           const bf16* __restrict__ d_out, G* __restrict__ d_table, int n, int C, int V) {
+// VEC elements per thread and access: 8 where rows are whole 16-byte vectors, else 2, or 1 for bases off a 4-byte boundary.  On B200, 4096 x
+// 1022 in vectors of 2 @N2@ us (297 us in a kernel with one row in flight, 330 us through copies padded to 8).
+constexpr int EMB_COLS = 512, EMB_AHEAD = 8;
+template <int VEC> struct alignas(VEC * 2) BfVec { bf16 v[VEC]; };
+template <typename G, int VEC>
+__global__ void __launch_bounds__(EMB_COLS / VEC) embedding_bwd_sorted_kernel(const int* __restrict__ sorted_ids, const long long* __restrict__ order,
+                                                                              const bf16* __restrict__ d_out, G* __restrict__ d_table, int n, int C, int V) {
     const int i = blockIdx.x;
     const int id = sorted_ids[i];
     if (id < 0 || id >= V || (i > 0 && sorted_ids[i - 1] == id)) return;
-    const int c = blockIdx.y * EMB_COLS + threadIdx.x * 8;
+    const int c = blockIdx.y * EMB_COLS + threadIdx.x * VEC;
     if (c >= C) return;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    using Vec = BfVec<VEC>;
+    float acc[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
     for (int j = i;; j += EMB_AHEAD) {
         bool mine[EMB_AHEAD];
         long long src[EMB_AHEAD];
@@ -599,30 +605,27 @@ __global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_sorted_kernel(const
             mine[u] = j + u < n && sorted_ids[j + u] == id;       // sorted: once false, false from there on
             src[u] = mine[u] ? order[j + u] : 0;
         }
-        uint4 raw[EMB_AHEAD];
+        Vec raw[EMB_AHEAD];
 #pragma unroll
         for (int u = 0; u < EMB_AHEAD; ++u)
-            if (mine[u]) raw[u] = *reinterpret_cast<const uint4*>(d_out + static_cast<size_t>(src[u]) * C + c);
+            if (mine[u]) raw[u] = *reinterpret_cast<const Vec*>(d_out + static_cast<size_t>(src[u]) * C + c);
 #pragma unroll
         for (int u = 0; u < EMB_AHEAD; ++u)
             if (mine[u]) {
-                float f[8];
-                unpack8(raw[u], f);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] += f[k];
+                for (int k = 0; k < VEC; ++k) acc[k] += __bfloat162float(raw[u].v[k]);
             }
         if (!mine[EMB_AHEAD - 1]) break;
     }
     G* dst = d_table + static_cast<size_t>(id) * C + c;
     if constexpr (sizeof(G) == 2) {
-        float o[8];
-        load8(reinterpret_cast<const bf16*>(dst), o);
+        Vec o = *reinterpret_cast<const Vec*>(dst);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] += acc[k];
-        store8(reinterpret_cast<bf16*>(dst), o);
+        for (int k = 0; k < VEC; ++k) o.v[k] = __float2bfloat16_rn(__bfloat162float(o.v[k]) + acc[k]);
+        *reinterpret_cast<Vec*>(dst) = o;
     } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dst[k] += acc[k];
+        for (int k = 0; k < VEC; ++k) dst[k] += acc[k];
     }
 }
 
@@ -1164,12 +1167,14 @@ void embedding_bwd(const int* tokens, const void* d_out, void* d_table, int grad
     if (grad_fp32) embedding_bwd_kernel<float><<<grid, 256, 0, s>>>(tokens, (const bf16*)d_out, (float*)d_table, n, C);
     else embedding_bwd_kernel<bf16><<<grid, 256, 0, s>>>(tokens, (const bf16*)d_out, (bf16*)d_table, n, C);
 }
-void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V,
+void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V, int vec,
                           cudaStream_t s) {
     if (n <= 0) return;
     const dim3 grid(n, (C + EMB_COLS - 1) / EMB_COLS);
-    if (grad_fp32) embedding_bwd_sorted_kernel<float><<<grid, EMB_THREADS, 0, s>>>(sorted_ids, order, (const bf16*)d_out, (float*)d_table, n, C, V);
-    else embedding_bwd_sorted_kernel<bf16><<<grid, EMB_THREADS, 0, s>>>(sorted_ids, order, (const bf16*)d_out, (bf16*)d_table, n, C, V);
+#define SG_EB(G, VEC) embedding_bwd_sorted_kernel<G, VEC><<<grid, EMB_COLS / VEC, 0, s>>>(sorted_ids, order, (const bf16*)d_out, (G*)d_table, n, C, V)
+    if (grad_fp32) { if (vec == 8) SG_EB(float, 8); else if (vec == 2) SG_EB(float, 2); else SG_EB(float, 1); }
+    else { if (vec == 8) SG_EB(bf16, 8); else if (vec == 2) SG_EB(bf16, 2); else SG_EB(bf16, 1); }
+#undef SG_EB
 }
 void zero_fill(void* p, size_t bytes, int num_sms, cudaStream_t s) { zero_fill_kernel<<<grid_for(bytes / 16, 256, num_sms), 256, 0, s>>>((uint4*)p, bytes / 16); }
 void cross_entropy_fwd_bwd(void* logits, const int* targets, float* loss, const float* scale_ptr, float scale_host, int rows, int V, int ld,

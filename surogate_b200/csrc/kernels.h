@@ -27,7 +27,8 @@ void qk_norm_rope_bwd(const void* d_out, const void* qkv_pre, const void* qw, co
 void embedding_fwd(const int* tokens, const void* table, void* out, size_t n, int C, int V, int* error_flag, int num_sms, cudaStream_t s);
 void embedding_bwd(const int* tokens, const void* d_out, void* d_table, int grad_fp32, size_t n, int C, int num_sms, cudaStream_t s);
 void zero_fill(void* p, size_t bytes, int num_sms, cudaStream_t s);   // 16-byte aligned, a multiple of 16
-void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V,
+// vec: elements per access, 8, 2 or 1; divides C, and d_out and d_table are aligned to vec bf16 elements
+void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V, int vec,
                           cudaStream_t s);
 void dequantize_fp8(const void* q, const float* scale, void* out, size_t n, int e5m2, int num_sms, cudaStream_t s);
 void cross_entropy_fwd_bwd_fp8(const void* logits, void* d8, const float* q_scale, const int* targets, float* loss, const float* scale_ptr, float scale_host, int rows,

@@ -333,6 +333,30 @@ def test_embedding_gradient_runs(ext, n, V, C, dt):
     assert not t.any()
 
 
+@pytest.mark.parametrize("C,shift", [(1022, 0), (510, 0), (512, 1), (520, 2), (6, 0)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_embedding_gradient_of_narrow_rows_needs_no_copy_of_the_table(ext, C, shift, dt):
+    """Rows that are not whole 16-byte vectors (even widths, views off the boundary) are summed in place: the bits of the aligned case, and
+    no allocation that grows with the table."""
+    torch.manual_seed(C)
+    n, V = 300, 20000
+    ids = torch.randint(0, 40, (n,), device=DEV, dtype=torch.int32)
+    d0 = torch.randn(n, C, device=DEV).bfloat16()
+    d = torch.empty(n * C + 8, device=DEV, dtype=torch.bfloat16)[shift:shift + n * C].view(n, C).copy_(d0)
+    start = torch.randn(V, C, device=DEV).to(dt)
+    pad = (C + 7) // 8 * 8 - C
+    want, rows = torch.nn.functional.pad(start, (0, pad)), torch.nn.functional.pad(d0, (0, pad))
+    ext.embedding_bwd(ids, rows, want)
+    got = torch.empty(V * C + 8, device=DEV, dtype=dt)[shift:shift + V * C].view(V, C).copy_(start)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    ext.embedding_bwd(ids, d, got)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want[:, :C])
+    assert torch.cuda.max_memory_allocated() - before < min(V * C, 1 << 20)
+
+
 @pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
 @pytest.mark.parametrize("e5m2", [False, True])
 def test_quantize_fp8_counts(ext, n, e5m2):
