@@ -3,9 +3,10 @@
 // One kernel template serves both passes.  A CTA keeps a RESIDENT pair of 128-row tiles and streams 64-row tile pairs through
 // a 4-stage TMA ring; the gradient accumulators stay in TMEM for the whole CTA.
 //   dK/dV pass: resident (K, V) of one 128-key tile of one KV head, streamed (Q, dO) tiles of the G query heads that share it:
-//               X = S^T, Y = dP^T, P^T = exp2(S^T - lse), dS^T = P^T o (dP^T - delta); dV += P^T dO, dK += dS^T Q.
-//   dQ pass   : resident (Q, dO) of one 128-query tile, streamed (K, V) tiles: X = S, Y = dP, dS = P o (dP - delta); dQ += dS K.
-// The softmax scale is applied once, to the finished dK / dQ.
+//               X = S^T, Y = dP^T, P^T = exp2(S^T - lse), dS^T = P^T o (dP^T - delta) scale; dV += P^T dO, dK += dS^T Q.
+//   dQ pass   : resident (Q, dO) of one 128-query tile, streamed (K, V) tiles: X = S, Y = dP, dS = P o (dP - delta) scale; dQ += dS K.
+// dS is scaled before it is rounded to bf16: scaling the finished dK / dQ instead saved nothing (the softmax warps wait for the tensor pipe) and
+// its error against fp64 was 0.2-0.8 % larger over four shapes.
 //
 // Two groups of four softmax warps take alternate items.  Each group has its own pair of score accumulators (X, Y) in TMEM, reads them,
 // and writes P and dS as bf16 over them, from where the accumulating MMAs take their A operand: no copy in shared memory, no proxy
@@ -62,7 +63,7 @@ struct Params {
     } while (0)
 
 // columns [64*half, 64*half+64) of a finished 128x128 fp32 accumulator -> bf16 row in global memory
-__device__ __forceinline__ void store_acc128(uint32_t t_acc, uint32_t lane_sel, __nv_bfloat16* dst_row, int half, float scale) {
+__device__ __forceinline__ void store_acc128(uint32_t t_acc, uint32_t lane_sel, __nv_bfloat16* dst_row, int half) {
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
         const int c = half * 2 + cc;
@@ -74,7 +75,7 @@ __device__ __forceinline__ void store_acc128(uint32_t t_acc, uint32_t lane_sel, 
             uint4 o;
             __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(__uint_as_float(raw[u * 8 + 2 * i]) * scale, __uint_as_float(raw[u * 8 + 2 * i + 1]) * scale);
+            for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(__uint_as_float(raw[u * 8 + 2 * i]), __uint_as_float(raw[u * 8 + 2 * i + 1]));
             *reinterpret_cast<uint4*>(dst_row + c * 32 + u * 8) = o;
         }
     }
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
             row_dl = p.delta[idx];
             if (HAS_LO) row_lo = __ldg(p.lo + row0 + row_abs);
         }
-        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), ds_scale2 = make_float2(p.scale, p.scale);
         bool ok = true;
         const bool do_prof = p.prof != nullptr && threadIdx.x == 64 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
         long long acc_[6] = {0, 0, 0, 0, 0, 0};
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
                         const float2 e = fma2(make_float2(__uint_as_float(x[c + k]), __uint_as_float(x[c + k + 1])), scale2, k ? make_float2(nl.z, nl.w) : make_float2(nl.x, nl.y));
                         const float2 pr = make_float2(ex2_approx(e.x), ex2_approx(e.y));
                         const float2 nd = k ? make_float2(-d4.z, -d4.w) : make_float2(-d4.x, -d4.y);
-                        const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(y[c + k]), __uint_as_float(y[c + k + 1])), nd));
+                        const float2 ds = mul2(mul2(pr, add2(make_float2(__uint_as_float(y[c + k]), __uint_as_float(y[c + k + 1])), nd)), ds_scale2);
                         const __nv_bfloat162 hp = __floats2bfloat162_rn(pr.x, pr.y), hs = __floats2bfloat162_rn(ds.x, ds.y);
                         if (!IS_DQ) pb[hf * 16 + (c + k) / 2] = reinterpret_cast<const uint32_t&>(hp);
                         sb[hf * 16 + (c + k) / 2] = reinterpret_cast<const uint32_t&>(hs);
@@ -313,10 +314,10 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
             const size_t width = static_cast<size_t>(p.Hq + 2 * p.Hkv) * D;
             __nv_bfloat16* base = p.d_qkv + static_cast<size_t>(row0 + row_abs) * width;
             if (IS_DQ) {
-                store_acc128(t_a1, lane_sel, base + head * D, group, p.scale);
+                store_acc128(t_a1, lane_sel, base + head * D, group);
             } else {
-                store_acc128(t_a1, lane_sel, base + kcol, group, p.scale);
-                store_acc128(t_a2, lane_sel, base + vcol, group, 1.f);
+                store_acc128(t_a1, lane_sel, base + kcol, group);
+                store_acc128(t_a2, lane_sel, base + vcol, group);
             }
         }
     }

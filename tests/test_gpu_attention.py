@@ -186,6 +186,33 @@ def test_flash_attention_backward_takes_a_misaligned_output(shift):
     check_device_errors()
 
 
+@pytest.mark.parametrize("t", [255, 130, 40])
+def test_flash_attention_backward_rounds_the_scaled_score_gradient(t):
+    """With K = 0 every score is zero and P = 1 / (t + 1); with d_out in query t alone and Q[t] = 1, dK[k] is the one score gradient of (t, k)
+    as the kernel hands it to the MMA: scale * P * (dP - delta), rounded to bf16 once.  A second rounding (of the unscaled value) would
+    change about a quarter of them; fp32 noise moves those within 2^-14 of a rounding boundary, below 2 % of them."""
+    from surogate_b200.ops import check_device_errors, ext
+
+    e = ext()
+    torch.manual_seed(t)
+    T, scale = 256, D ** -0.5
+    qkv = torch.randn(1, T, 3 * D, device=DEV).bfloat16()
+    qkv[..., D:2 * D] = 0
+    qkv[0, t, :D] = 1
+    out, lse = e.flash_attn_fwd(qkv, 1, 1, scale, None)
+    d_out = torch.zeros_like(out)
+    d_out[0, t] = torch.randn(D, device=DEV).bfloat16()
+    dk = e.flash_attn_bwd(d_out, qkv, out, lse, 1, 1, scale, None, None)[0, :t + 1, D:2 * D]
+    torch.cuda.synchronize()
+    check_device_errors()
+    g = d_out[0, t].double()
+    ds = (qkv[0, :t + 1, 2 * D:].double() @ g - out[0, t].double() @ g) * torch.exp(-lse[0, t, 0].double())
+    assert torch.equal(dk, dk[:, :1].expand_as(dk))
+    wrong = (dk[:, 0] != (scale * ds).float().bfloat16()).float().mean().item()
+    twice = (dk[:, 0] != (scale * ds.float().bfloat16().double()).float().bfloat16()).float().mean().item()
+    assert wrong <= 0.02 + 1.0 / (t + 1) < twice, (wrong, twice)
+
+
 def test_packed_batch_trains_like_the_masked_fp32_path():
     """One packed batch (position ids reset inside the rows) and one sliding-window model through the trainer on the CUDA backend:
     loss and gradient norm equal the PyTorch backend, whose attention applies the explicit document / window mask."""
