@@ -582,9 +582,14 @@ template <typename G> __global__ void embedding_bwd_kernel(const int* __restrict
 // the first is added, and the columns are spread over CTAs.  8192 rows of 4096, longest run 160, on B200: 577 -> 166 us with the sort
 // (about 100 us of it).
 // VEC elements per thread and access: 8 where rows are whole 16-byte vectors, else 2, or 1 for bases off a 4-byte boundary.  On B200, 4096 x
-// 1022 in vectors of 2 @N2@ us (297 us in a kernel with one row in flight, 330 us through copies padded to 8).
+// 1022 in vectors of 2 147 us (297 us in a kernel with one row in flight, 330 us through copies padded to 8).
 constexpr int EMB_COLS = 512, EMB_AHEAD = 8;
-template <int VEC> struct alignas(VEC * 2) BfVec { bf16 v[VEC]; };
+template <int VEC> struct EmbWord { using T = uint4; };
+template <> struct EmbWord<2> { using T = uint32_t; };
+template <> struct EmbWord<1> { using T = unsigned short; };
+__device__ __forceinline__ void emb_unpack(const uint4& w, float (&f)[8]) { unpack8(w, f); }
+__device__ __forceinline__ void emb_unpack(const uint32_t& w, float (&f)[2]) { f[0] = __uint_as_float(w << 16); f[1] = __uint_as_float(w & 0xFFFF0000u); }
+__device__ __forceinline__ void emb_unpack(const unsigned short& w, float (&f)[1]) { f[0] = __uint_as_float(static_cast<uint32_t>(w) << 16); }
 template <typename G, int VEC>
 __global__ void __launch_bounds__(EMB_COLS / VEC) embedding_bwd_sorted_kernel(const int* __restrict__ sorted_ids, const long long* __restrict__ order,
                                                                               const bf16* __restrict__ d_out, G* __restrict__ d_table, int n, int C, int V) {
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(EMB_COLS / VEC) embedding_bwd_sorted_kernel(co
     if (id < 0 || id >= V || (i > 0 && sorted_ids[i - 1] == id)) return;
     const int c = blockIdx.y * EMB_COLS + threadIdx.x * VEC;
     if (c >= C) return;
-    using Vec = BfVec<VEC>;
+    using Word = typename EmbWord<VEC>::T;
     float acc[VEC];
 #pragma unroll
     for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
@@ -605,24 +610,35 @@ __global__ void __launch_bounds__(EMB_COLS / VEC) embedding_bwd_sorted_kernel(co
             mine[u] = j + u < n && sorted_ids[j + u] == id;       // sorted: once false, false from there on
             src[u] = mine[u] ? order[j + u] : 0;
         }
-        Vec raw[EMB_AHEAD];
+        Word raw[EMB_AHEAD];
 #pragma unroll
         for (int u = 0; u < EMB_AHEAD; ++u)
-            if (mine[u]) raw[u] = *reinterpret_cast<const Vec*>(d_out + static_cast<size_t>(src[u]) * C + c);
+            if (mine[u]) raw[u] = *reinterpret_cast<const Word*>(d_out + static_cast<size_t>(src[u]) * C + c);
 #pragma unroll
         for (int u = 0; u < EMB_AHEAD; ++u)
             if (mine[u]) {
+                float f[VEC];
+                emb_unpack(raw[u], f);
 #pragma unroll
-                for (int k = 0; k < VEC; ++k) acc[k] += __bfloat162float(raw[u].v[k]);
+                for (int k = 0; k < VEC; ++k) acc[k] += f[k];
             }
         if (!mine[EMB_AHEAD - 1]) break;
     }
     G* dst = d_table + static_cast<size_t>(id) * C + c;
     if constexpr (sizeof(G) == 2) {
-        Vec o = *reinterpret_cast<const Vec*>(dst);
+        float o[VEC];
+        emb_unpack(*reinterpret_cast<const Word*>(dst), o);
+        alignas(16) bf16 r[VEC];
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) o.v[k] = __float2bfloat16_rn(__bfloat162float(o.v[k]) + acc[k]);
-        *reinterpret_cast<Vec*>(dst) = o;
+        for (int k = 0; k < VEC; ++k) r[k] = __float2bfloat16_rn(o[k] + acc[k]);
+        *reinterpret_cast<Word*>(dst) = *reinterpret_cast<const Word*>(r);
+    } else if constexpr (VEC == 8) {
+#pragma unroll
+        for (int k = 0; k < VEC; k += 4) {
+            float4 o = *reinterpret_cast<const float4*>(dst + k);
+            o.x += acc[k]; o.y += acc[k + 1]; o.z += acc[k + 2]; o.w += acc[k + 3];
+            *reinterpret_cast<float4*>(dst + k) = o;
+        }
     } else {
 #pragma unroll
         for (int k = 0; k < VEC; ++k) dst[k] += acc[k];

@@ -353,8 +353,9 @@ def test_embedding_gradient_of_narrow_rows_needs_no_copy_of_the_table(ext, C, sh
     before = torch.cuda.memory_allocated()
     ext.embedding_bwd(ids, d, got)
     torch.cuda.synchronize()
+    grown = torch.cuda.max_memory_allocated() - before
     assert torch.equal(got, want[:, :C])
-    assert torch.cuda.max_memory_allocated() - before < min(V * C, 1 << 20)
+    assert grown < min(V * C, 1 << 20)       # the sort of the ids: a few KB for each
 
 
 @pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
