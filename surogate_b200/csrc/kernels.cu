@@ -358,12 +358,15 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict_
 // ------------------------------------------------------------------------------------------ QK-norm + RoPE
 // Half a warp per (token, head); head_dim 128: lane s = lane & 15 of the half holds elements [8s, 8s+8) (one 16-byte access), the
 // rotary partner (i +/- 64) lives in lane s ^ 8 of the same half.  A warp works on one token at a time and walks all of its heads,
-// two at a time (one per half-warp).  A block takes eight tokens at a time; its threads evaluate the sines and cosines of all of them
-// together, each angle once, into shared memory (two tables in turn, so one barrier per eight tokens).  Evaluated in every lane that uses
-// them they cost four times the work and the registers of a third resident block.  On B200 forward 2 x 4096 x 48 heads 67 -> 61 us, 3 x 1000 x 32 heads 26 -> 21 us;
-// backward 101 -> 99 and 50 -> 47 us.
+// two at a time (one per half-warp).  A block takes eight tokens at a time (forward: four, two warps to a token); its threads evaluate the
+// sines and cosines of all of them together, each angle once, into shared memory (two tables in turn, so one barrier per group of tokens).
+// Evaluated in every lane that uses them they cost four times the work and the registers of a third resident block.  Eight tokens to a
+// block of the forward left a second wave of few blocks at 4096 tokens.  On B200, in L2, with angles per lane -> eight tokens -> four,
+// 2 x 2048 x 48 heads 31.3 -> 33.1 -> 30.3 us,
+// 2 x 4096 x 48 61.8 -> 53.7 -> 54.2, 1 x 1000 x 32 8.5 -> 8.6 -> 7.0; backward (eight) 95.3 -> 93.0 us at 2 x 4096 x 48.
 // Layout per token: [Hq heads | Hkv heads (K) | Hkv heads (V)] x D.  V heads are copied (forward) / passed through (backward).
 constexpr int ROPE_PAIRS_IN_FLIGHT = 4;      // head pairs whose loads are issued before the first is used
+constexpr int rope_tokens(bool backward) { return backward ? 8 : 4; }
 __device__ __forceinline__ float half_warp_sum(float v) {
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -381,7 +384,8 @@ __global__ void __launch_bounds__(256, BACKWARD ? 2 : 3) qk_norm_rope_kernel(con
     constexpr int D = 128;
     constexpr int U = ROPE_PAIRS_IN_FLIGHT;
     __shared__ float sdw[2][D];
-    __shared__ alignas(16) float trig[2][8][2][D / 2];     // [table][warp's token][cos | sin][frequency]
+    constexpr int TOK = rope_tokens(BACKWARD), WPT = 8 / TOK;     // tokens of a block, warps per token
+    __shared__ alignas(16) float trig[2][TOK][2][D / 2];   // [table][token][cos | sin][frequency]
     const bool multi_axis = (lim_h | lim_w) != 0;
     if (BACKWARD) {
         for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&sdw[0][0])[i] = 0.f;
@@ -404,15 +408,15 @@ __global__ void __launch_bounds__(256, BACKWARD ? 2 : 3) qk_norm_rope_kernel(con
         dw_acc[0][i] = 0.f;
         dw_acc[1][i] = 0.f;
     }
-    // the frequency whose angles this thread evaluates, for tokens threadIdx.x / 64 and + 4 of the block's eight
+    // the frequency whose angles this thread evaluates, for tokens threadIdx.x / 64 (and + 4) of the block's
     const int freq = threadIdx.x & 63, m3 = freq % 3;
     const float inv = exp2f(-log2_theta * (2.f * freq) / D);
     const size_t axis_row = (m3 == 1 && freq < lim_h) ? tokens : ((m3 == 2 && freq < lim_w) ? 2 * tokens : 0);
     const float sign = (sub < 8) ? -1.f : 1.f;  // first half of the head: x1*c - x2*s ; second half: x2*c + x1*s
     int table = 0;
-    for (size_t tok0 = static_cast<size_t>(blockIdx.x) * 8; tok0 < tokens; tok0 += static_cast<size_t>(gridDim.x) * 8, table ^= 1) {
+    for (size_t tok0 = static_cast<size_t>(blockIdx.x) * TOK; tok0 < tokens; tok0 += static_cast<size_t>(gridDim.x) * TOK, table ^= 1) {
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < TOK / 4; ++k) {
             const int w = (threadIdx.x >> 6) + 4 * k;
             if (tok0 + w < tokens) {
                 float sn, cs;
@@ -422,15 +426,16 @@ __global__ void __launch_bounds__(256, BACKWARD ? 2 : 3) qk_norm_rope_kernel(con
             }
         }
         __syncthreads();
-        const size_t tok = tok0 + warp;
+        const int slot = warp / WPT;
+        const size_t tok = tok0 + slot;
         if (tok >= tokens) continue;
         float cs[8], sn[8];
-        *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(&trig[table][warp][0][(sub & 7) * 8]);
-        *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(&trig[table][warp][0][(sub & 7) * 8 + 4]);
-        *reinterpret_cast<float4*>(sn) = *reinterpret_cast<const float4*>(&trig[table][warp][1][(sub & 7) * 8]);
-        *reinterpret_cast<float4*>(sn + 4) = *reinterpret_cast<const float4*>(&trig[table][warp][1][(sub & 7) * 8 + 4]);
+        *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(&trig[table][slot][0][(sub & 7) * 8]);
+        *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(&trig[table][slot][0][(sub & 7) * 8 + 4]);
+        *reinterpret_cast<float4*>(sn) = *reinterpret_cast<const float4*>(&trig[table][slot][1][(sub & 7) * 8]);
+        *reinterpret_cast<float4*>(sn + 4) = *reinterpret_cast<const float4*>(&trig[table][slot][1][(sub & 7) * 8 + 4]);
         const size_t tbase = tok * static_cast<size_t>(H) * D + sub * 8;
-        for (int hb = 0; hb < H; hb += 2 * U) {
+        for (int hb = (warp % WPT) * 2 * U; hb < H; hb += 2 * U * WPT) {
             // all loads of this batch of head pairs are issued before any of them is used
             uint4 raws[U], pres[U];
 #pragma unroll
@@ -1164,14 +1169,14 @@ void zero_empty_groups(void* out, const int* offsets, int groups, size_t bytes_p
 }
 void qk_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, const int* pos, void* out, float* q_rstd, float* k_rstd, size_t tokens, int Hq,
                       int Hkv, float eps, float theta, int lim_h, int lim_w, int num_sms, cudaStream_t s) {
-    qk_norm_rope_kernel<false><<<grid_for(tokens * 32, 256, num_sms, 8), 256, 0, s>>>((const bf16*)qkv, nullptr, (const bf16*)qw, (const bf16*)kw, pos,
+    qk_norm_rope_kernel<false><<<grid_for(tokens, rope_tokens(false), num_sms, 16), 256, 0, s>>>((const bf16*)qkv, nullptr, (const bf16*)qw, (const bf16*)kw, pos,
                                                                                    (bf16*)out, q_rstd, k_rstd, nullptr, nullptr, tokens, Hq, Hkv, eps,
                                                                                    log2f(theta), lim_h, lim_w);
 }
 void qk_norm_rope_bwd(const void* d_out, const void* qkv_pre, const void* qw, const void* kw, const int* pos, void* d_qkv, float* q_rstd,
                       float* k_rstd, float* dqw, float* dkw, size_t tokens, int Hq, int Hkv, float eps, float theta, int lim_h, int lim_w, int num_sms,
                       cudaStream_t s) {
-    qk_norm_rope_kernel<true><<<grid_for(tokens * 32, 256, num_sms, 4), 256, 0, s>>>((const bf16*)d_out, (const bf16*)qkv_pre, (const bf16*)qw,
+    qk_norm_rope_kernel<true><<<grid_for(tokens, rope_tokens(true), num_sms, 4), 256, 0, s>>>((const bf16*)d_out, (const bf16*)qkv_pre, (const bf16*)qw,
                                                                                      (const bf16*)kw, pos, (bf16*)d_qkv, q_rstd, k_rstd, dqw, dkw, tokens,
                                                                                      Hq, Hkv, eps, log2f(theta), lim_h, lim_w);
 }
