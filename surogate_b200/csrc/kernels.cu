@@ -929,12 +929,15 @@ __device__ __forceinline__ float rcp_fast(float x) {
 __device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
 constexpr float kRoundMagic = 12582912.f;   // 1.5 * 2^23: adding it rounds to the nearest integer and leaves it in the low mantissa bits
 
-// Weights, gradients and codes reach the registers through a ring of ADAM8_STAGES shared-memory slots (cp.async; every thread copies and
+// Weights, gradients and codes reach the registers through a ring of shared-memory slots (cp.async; every thread copies and
 // reads only its own 8 elements, so the ring needs no barrier): three trips' worth of loads are outstanding while one is computed, 110 KB
 // per SM.  The group scales are two bytes each, below what cp.async moves, and are fetched one trip ahead into registers.  With loads and
 // arithmetic of a trip one after the other, DRAM idled during the arithmetic of all three CTAs: 64 M parameters in bf16
 // on B200 167 -> 141 us (4.9 TB/s).
-constexpr int ADAM8_STAGES = 4, ADAM8_THREADS = 256;
+// Four slots, or three where weights and gradients are both fp32: four of those leave room for two CTAs per SM only, and then the arithmetic
+// is short of warps (64 M parameters 183 us with loads and arithmetic in turn, 195 with four slots, 169 with three).
+constexpr int ADAM8_THREADS = 256;
+template <typename P, typename G> constexpr int adam8_stages() { return sizeof(P) + sizeof(G) >= 8 ? 3 : 4; }
 template <typename P, typename G> constexpr int adam8_slot_bytes() { return ADAM8_THREADS * (8 * static_cast<int>(sizeof(P) + sizeof(G)) + 16); }
 template <int BYTES> __device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
     if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -960,7 +963,7 @@ __global__ void __launch_bounds__(ADAM8_THREADS, 3) adamw_8bit_kernel(P* __restr
     const float decay_on = 1.f - lr * wd;
     const char* lut_bytes = reinterpret_cast<const char*>(m_lut);
     const size_t nvec = n / 8;
-    constexpr int PB = 8 * sizeof(P), GB = 8 * sizeof(G), SLOT = adam8_slot_bytes<P, G>();
+    constexpr int PB = 8 * sizeof(P), GB = 8 * sizeof(G), SLOT = adam8_slot_bytes<P, G>(), STAGES = adam8_stages<P, G>();
     constexpr int OFF_G = ADAM8_THREADS * PB, OFF_M = OFF_G + ADAM8_THREADS * GB, OFF_V = OFF_M + ADAM8_THREADS * 8;
     const uint32_t ring0 = smem_u32(ring);
     const size_t stride = static_cast<size_t>(gridDim.x) * ADAM8_THREADS;
@@ -978,7 +981,7 @@ __global__ void __launch_bounds__(ADAM8_THREADS, 3) adamw_8bit_kernel(P* __restr
     };
     const size_t first = blockIdx.x * static_cast<size_t>(ADAM8_THREADS) + threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < ADAM8_STAGES - 1; ++k) request(first + k * stride, k);
+    for (int k = 0; k < STAGES - 1; ++k) request(first + k * stride, k);
     uint2 next_mk = make_uint2(0x01010101u, 0x01010101u);
     float next_sm = 0.f, next_sq = 0.f;
     auto fetch_scales = [&](size_t vi) {
@@ -997,13 +1000,13 @@ __global__ void __launch_bounds__(ADAM8_THREADS, 3) adamw_8bit_kernel(P* __restr
     for (size_t base = blockIdx.x * static_cast<size_t>(ADAM8_THREADS) + (threadIdx.x & ~31); base < nvec; base += stride) {
         const size_t vi = base + (threadIdx.x & 31), idx = vi * 8;
         const bool live = vi < nvec;
-        request(vi + (ADAM8_STAGES - 1) * stride, (slot + ADAM8_STAGES - 1) % ADAM8_STAGES);   // the slot that the previous trip emptied
+        request(vi + (STAGES - 1) * stride, (slot + STAGES - 1) % STAGES);   // the slot that the previous trip emptied
         const uint2 mk = next_mk;
         const float sm = next_sm, sq = next_sq;
         fetch_scales(vi + stride);
-        asm volatile("cp.async.wait_group %0;" ::"n"(ADAM8_STAGES - 1) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
         const uint8_t* cell = ring + slot * SLOT;
-        slot = slot + 1 == ADAM8_STAGES ? 0 : slot + 1;
+        slot = slot + 1 == STAGES ? 0 : slot + 1;
         {
             float pv[8], gv[8];
             load8_any(reinterpret_cast<const P*>(cell + threadIdx.x * PB), pv);
@@ -1240,9 +1243,10 @@ void adamw_8bit(void* p, int p_fp32, const void* g, int g_fp32, void* m8, void* 
                 const float* hp, size_t n, int num_sms, cudaStream_t s) {
 #define SG_A8(PT, GT, BM)                                                                                                                       \
     do {                                                                                                                                        \
-        constexpr int smem = ADAM8_STAGES * adam8_slot_bytes<PT, GT>();                                                                           \
+        constexpr int smem = adam8_stages<PT, GT>() * adam8_slot_bytes<PT, GT>();                                                                 \
+        static_assert(3 * (smem + 2048) <= 227 * 1024, "three CTAs per SM");                                                                     \
         cudaFuncSetAttribute(adamw_8bit_kernel<PT, GT, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   /* of the current device */        \
-        const int grid = grid_for(n / 8, ADAM8_THREADS, num_sms, smem > 72 * 1024 ? 2 : 3);   /* the resident CTAs, each with a full ring */      \
+        const int grid = grid_for(n / 8, ADAM8_THREADS, num_sms, 3);   /* the resident CTAs, each with a full ring */      \
         adamw_8bit_kernel<PT, GT, BM><<<grid, ADAM8_THREADS, smem, s>>>((PT*)p, (const GT*)g, (int8_t*)m8, (uint8_t*)v8, (__half*)ms, (__half*)vs, mask, hp, n); \
     } while (0)
     if (block_mask) {
