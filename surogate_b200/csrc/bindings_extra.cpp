@@ -372,7 +372,7 @@ std::vector<Tensor> nvfp4_quantize_transpose(const Tensor& x, const Tensor& amax
     Tensor sf = torch::empty({nvfp4_sf_bytes(C, R)}, x.options().dtype(at::kByte));
     sg_count_launch(1);
     sg::nvfp4_quantize_transpose(x.data_ptr(), q.data_ptr(), sf.data_ptr(), amax.data_ptr<float>(), R, C, stochastic, hadamard,
-                                 static_cast<uint32_t>(seed), static_cast<uint32_t>(sign_mask), cur_stream(), four_over_six && !stochastic);
+                                 static_cast<uint32_t>(seed), static_cast<uint32_t>(sign_mask), sms(), cur_stream(), four_over_six && !stochastic);
     return {q, sf};
 }
 

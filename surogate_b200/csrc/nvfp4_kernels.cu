@@ -175,9 +175,11 @@ __device__ __forceinline__ void hadamard16(float (&v)[16], uint32_t sign_mask) {
 // Both quantisers work on tiles of 128 output rows x 128 elements (8 blocks of 16): the codes (64 bytes a row) and the scales (two
 // 512-byte atoms) are collected in shared memory and leave as whole sectors.  Written straight from the threads that compute them, each
 // scale is a one-byte store into a sector of its own, and the codes of a transpose are 8-byte stores a whole row apart.
-constexpr int QT_ROWS = 128, QT_COLS = 128, QT_BLOCKS = QT_COLS / 16, QT_PITCH = QT_COLS / 2 + 8;
-struct QTile {
-    uint8_t q[QT_ROWS * QT_PITCH];
+// Stochastic rounding issues about 500 instructions per block of 16, so a tensor of few tiles is bound by the SMs that it occupies: with at
+// most one tile per SM, tiles are cut into QT_FEW_ROWS rows (each a quarter of the words of its two atoms).
+constexpr int QT_ROWS = 128, QT_FEW_ROWS = 32, QT_COLS = 128, QT_BLOCKS = QT_COLS / 16, QT_PITCH = QT_COLS / 2 + 8;
+template <int ROWS> struct QTile {
+    uint8_t q[ROWS * QT_PITCH];
     alignas(16) uint8_t sf[QT_ROWS * QT_BLOCKS];
     __device__ __forceinline__ void put(int r, int b, const uint32_t (&codes)[2], uint8_t scale) {
         *reinterpret_cast<uint2*>(q + r * QT_PITCH + b * 8) = make_uint2(codes[0], codes[1]);
@@ -186,14 +188,17 @@ struct QTile {
     // `rows` x `kblocks`: the whole output; (row0, kb0): this tile's origin.  Scales of rows and blocks behind the end are zero, so the
     // buffer needs no clearing beforehand.
     __device__ __forceinline__ void write(uint8_t* __restrict__ qg, uint8_t* __restrict__ sfg, int row0, int kb0, int rows, int kblocks, int atoms_k) const {
-        for (int i = threadIdx.x; i < QT_ROWS * QT_BLOCKS; i += blockDim.x) {
+        for (int i = threadIdx.x; i < ROWS * QT_BLOCKS; i += blockDim.x) {
             const int r = i / QT_BLOCKS, b = i % QT_BLOCKS;
             if (row0 + r < rows && kb0 + b < kblocks)
                 *reinterpret_cast<uint2*>(qg + (static_cast<size_t>(row0 + r) * kblocks + kb0 + b) * 8) = *reinterpret_cast<const uint2*>(q + r * QT_PITCH + b * 8);
         }
         const int atom0 = kb0 >> 2;
-        if (threadIdx.x < 64 && atom0 + (threadIdx.x >> 5) < atoms_k)
-            reinterpret_cast<uint4*>(sfg + (static_cast<size_t>(row0 >> 7) * atoms_k + atom0) * 512)[threadIdx.x] = reinterpret_cast<const uint4*>(sf)[threadIdx.x];
+        if (threadIdx.x < 64 && atom0 + (threadIdx.x >> 5) < atoms_k) {
+            uint4* atom = reinterpret_cast<uint4*>(sfg + (static_cast<size_t>(row0 >> 7) * atoms_k + atom0) * 512);
+            if (ROWS == QT_ROWS) atom[threadIdx.x] = reinterpret_cast<const uint4*>(sf)[threadIdx.x];
+            else reinterpret_cast<uint32_t*>(atom + threadIdx.x)[(row0 >> 5) & 3] = reinterpret_cast<const uint32_t*>(sf)[threadIdx.x * 4];
+        }
     }
 };
 
@@ -203,18 +208,19 @@ struct QTile {
 // candidates' codes and error sums), about 30 with stochastic rounding (the hash).  24576 x 4096 on B200: four-over-six 958 -> 95 us
 // (2.7 TB/s of the 258 MB it must move), plain 151 -> 64 us, stochastic 476 -> 197 us; before, the codes came from a chain of compares,
 // their values from a table in local memory, and every scale byte was a store of its own.
-template <bool SR>
+// Stochastic, 256 x 1024: scale bytes stored one by one 5.8 us, whole tiles 7.7 us, 32 rows 3.4 us.
+template <bool SR, int ROWS>
 __global__ void __launch_bounds__(256) nvfp4_quantize_rows_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                                   const float* __restrict__ amax_tensor, int rows, int K, int atoms_k, uint32_t seed,
                                                                   int block2d, int four_over_six) {
-    __shared__ QTile out_tile;
+    __shared__ QTile<ROWS> out_tile;
     const float at = __ldg(amax_tensor);
     const float ge = at > 0.f ? __fdiv_rn(four_over_six ? 1536.f : 2688.f, at) : 1.f;
     const int kblocks = K / 16;
     const int tiles_k = (kblocks + QT_BLOCKS - 1) / QT_BLOCKS;
-    const int row0 = static_cast<int>(blockIdx.x / tiles_k) * QT_ROWS, kb0 = static_cast<int>(blockIdx.x % tiles_k) * QT_BLOCKS;
+    const int row0 = static_cast<int>(blockIdx.x / tiles_k) * ROWS, kb0 = static_cast<int>(blockIdx.x % tiles_k) * QT_BLOCKS;
 #pragma unroll 1
-    for (int it = 0; it < QT_ROWS * QT_BLOCKS / 256; ++it) {
+    for (int it = 0; it < ROWS * QT_BLOCKS / 256; ++it) {
         int r, b;
         if (block2d) {   // lanes walk down the 16 rows of a 16x16 tile, so that its abs-max and its decision are 16-lane shuffles
             const int tile = it * 16 + (threadIdx.x >> 4);
@@ -253,18 +259,19 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_rows_kernel(const bf16* __
 // x [R, C] bf16 -> quantised x^T: q [C, R/2], sf for (row = c, block = r/16).  R % 64 == 0, C % 64 == 0.
 // The 128 x 128 input tile passes through shared memory as bf16; a lane owns two adjacent columns (4-byte reads, no bank conflicts).
 // 24576 x 4096 on B200: four-over-six 1284 -> 98 us, with the Hadamard transform 1316 -> 118 us, stochastic with it 349 -> 221 us.
-constexpr int QX_PITCH = QT_ROWS + 8;     // bf16 elements per staged row
-template <bool SR, bool RHT>
-__global__ void __launch_bounds__(256) nvfp4_quantize_transpose_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
+// Stochastic, 256 x 1024: 64 x 64 tiles 6.2 us, whole tiles 7.7 us, 32 rows 3.9 us.
+template <bool SR, bool RHT, int ROWS, int THREADS>
+__global__ void __launch_bounds__(THREADS) nvfp4_quantize_transpose_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                                        const float* __restrict__ amax_tensor, int R, int C, int atoms_k, uint32_t seed,
                                                                        uint32_t sign_mask, int four_over_six) {
-    __shared__ QTile out_tile;
+    constexpr int QX_PITCH = ROWS + 8;        // bf16 elements per staged row
+    __shared__ QTile<ROWS> out_tile;
     __shared__ alignas(16) bf16 tile[QT_COLS * QX_PITCH];
-    const int tiles_c = (C + QT_ROWS - 1) / QT_ROWS;
-    const int c0 = static_cast<int>(blockIdx.x % tiles_c) * QT_ROWS, r0 = static_cast<int>(blockIdx.x / tiles_c) * QT_COLS;
+    const int tiles_c = (C + QT_ROWS - 1) / QT_ROWS * (QT_ROWS / ROWS);
+    const int c0 = static_cast<int>(blockIdx.x % tiles_c) * ROWS, r0 = static_cast<int>(blockIdx.x / tiles_c) * QT_COLS;
 #pragma unroll
-    for (int it = 0; it < QT_COLS * QT_ROWS / 8 / 256; ++it) {
-        const int i = it * 256 + threadIdx.x, rr = i / (QT_ROWS / 8), cv = (i % (QT_ROWS / 8)) * 8;
+    for (int it = 0; it < QT_COLS * ROWS / 8 / THREADS; ++it) {
+        const int i = it * THREADS + threadIdx.x, rr = i / (ROWS / 8), cv = (i % (ROWS / 8)) * 8;
         uint4 raw = make_uint4(0, 0, 0, 0);
         if (r0 + rr < R && c0 + cv < C) raw = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r0 + rr) * C + c0 + cv);
         *reinterpret_cast<uint4*>(tile + rr * QX_PITCH + cv) = raw;
@@ -275,8 +282,8 @@ __global__ void __launch_bounds__(256) nvfp4_quantize_transpose_kernel(const bf1
     const float enc = (!SR && four_over_six) ? 1536.f : 2688.f;
     const float ge = at > 0.f ? (RHT ? enc / (at * 2.f) : enc / at) : 1.f;
 #pragma unroll 1
-    for (int it = 0; it < QT_ROWS / 2 * QT_BLOCKS / 256; ++it) {
-        const int i = it * 256 + threadIdx.x, pair = i % (QT_ROWS / 2), rb = i / (QT_ROWS / 2);   // columns 2 pair, 2 pair + 1; 16-row block
+    for (int it = 0; it < ROWS / 2 * QT_BLOCKS / THREADS; ++it) {
+        const int i = it * THREADS + threadIdx.x, pair = i % (ROWS / 2), rb = i / (ROWS / 2);   // columns 2 pair, 2 pair + 1; 16-row block
         bf162 raw[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) raw[k] = *reinterpret_cast<const bf162*>(tile + (rb * 16 + k) * QX_PITCH + 2 * pair);
@@ -327,24 +334,32 @@ static int q_grid(size_t items, int num_sms) {
 void nvfp4_quantize_rows(const void* x, void* q, void* sf, const float* amax_tensor, int rows, int K, int stochastic, uint32_t seed, int block2d,
                          int num_sms, cudaStream_t s, int four_over_six) {
     const int atoms_k = (K / 16 + 3) / 4;
-    (void)num_sms;
     if (rows <= 0 || K <= 0) return;
     const unsigned grid = static_cast<unsigned>((rows + QT_ROWS - 1) / QT_ROWS) * static_cast<unsigned>((K / 16 + QT_BLOCKS - 1) / QT_BLOCKS);
-    if (stochastic) nvfp4_quantize_rows_kernel<true><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, (uint8_t*)sf, amax_tensor, rows, K, atoms_k, seed, block2d, 0);
-    else nvfp4_quantize_rows_kernel<false><<<grid, 256, 0, s>>>((const bf16*)x, (uint8_t*)q, (uint8_t*)sf, amax_tensor, rows, K, atoms_k, seed, block2d, four_over_six);
+#define SG_QR(SR, ROWS, FOS)                                                                                                                            \
+    nvfp4_quantize_rows_kernel<SR, ROWS><<<grid * (QT_ROWS / ROWS), 256, 0, s>>>((const bf16*)x, (uint8_t*)q, (uint8_t*)sf, amax_tensor, rows, K, atoms_k, seed, \
+                                                                                 block2d, FOS)
+    if (stochastic && grid <= static_cast<unsigned>(num_sms)) SG_QR(true, QT_FEW_ROWS, 0);
+    else if (stochastic) SG_QR(true, QT_ROWS, 0);
+    else SG_QR(false, QT_ROWS, four_over_six);
+#undef SG_QR
 }
 void nvfp4_quantize_transpose(const void* x, void* q, void* sf, const float* amax_tensor, int R, int C, int stochastic, int hadamard, uint32_t seed,
-                              uint32_t sign_mask, cudaStream_t s, int four_over_six) {
+                              uint32_t sign_mask, int num_sms, cudaStream_t s, int four_over_six) {
     const int atoms_k = (R / 16 + 3) / 4;
     if (R <= 0 || C <= 0) return;
     const unsigned grid = static_cast<unsigned>((C + QT_ROWS - 1) / QT_ROWS) * static_cast<unsigned>((R + QT_COLS - 1) / QT_COLS);
     const bf16* xp = (const bf16*)x;
     uint8_t* qp = (uint8_t*)q;
     uint8_t* sp = (uint8_t*)sf;
-    if (stochastic && hadamard) nvfp4_quantize_transpose_kernel<true, true><<<grid, 256, 0, s>>>(xp, qp, sp, amax_tensor, R, C, atoms_k, seed, sign_mask, four_over_six);
-    else if (stochastic) nvfp4_quantize_transpose_kernel<true, false><<<grid, 256, 0, s>>>(xp, qp, sp, amax_tensor, R, C, atoms_k, seed, sign_mask, four_over_six);
-    else if (hadamard) nvfp4_quantize_transpose_kernel<false, true><<<grid, 256, 0, s>>>(xp, qp, sp, amax_tensor, R, C, atoms_k, seed, sign_mask, four_over_six);
-    else nvfp4_quantize_transpose_kernel<false, false><<<grid, 256, 0, s>>>(xp, qp, sp, amax_tensor, R, C, atoms_k, seed, sign_mask, four_over_six);
+#define SG_QX(SR, RHT, ROWS, TH)                                                                                                                        \
+    nvfp4_quantize_transpose_kernel<SR, RHT, ROWS, TH><<<grid * (QT_ROWS / ROWS), TH, 0, s>>>(xp, qp, sp, amax_tensor, R, C, atoms_k, seed, sign_mask, four_over_six)
+    const bool few = grid <= static_cast<unsigned>(num_sms);
+    if (stochastic && hadamard) { if (few) SG_QX(true, true, QT_FEW_ROWS, 128); else SG_QX(true, true, QT_ROWS, 256); }
+    else if (stochastic) { if (few) SG_QX(true, false, QT_FEW_ROWS, 128); else SG_QX(true, false, QT_ROWS, 256); }
+    else if (hadamard) SG_QX(false, true, QT_ROWS, 256);
+    else SG_QX(false, false, QT_ROWS, 256);
+#undef SG_QX
 }
 void nvfp4_dequantize(const void* q, const void* sf, const float* amax_tensor, float amax_div, void* out, int rows, int K, int num_sms, cudaStream_t s,
                       float encode) {

@@ -195,3 +195,27 @@ def test_quantisers_at_the_edges_of_their_tiles(ext, transpose, rows, K, stochas
         codes = torch.from_numpy(_sr_codes(s, 11, idx).astype(np.int64)).to(DEV)
     wrong = (ref.unpack_codes(q) != codes) & (~sf_bad).repeat_interleave(16, dim=1)
     assert wrong.float().mean().item() < 2e-3       # a product on a rounding boundary may fall the other way
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("hadamard", [False, True])
+def test_stochastic_codes_do_not_depend_on_the_tile_height(ext, transpose, hadamard):
+    """Tensors of at most one 128 x 128 tile per SM are quantised in tiles of 32 rows, larger ones in whole tiles (19 x 8 of them here): the same
+    codes and scales, since the random numbers belong to the element."""
+    if hadamard and not transpose:
+        pytest.skip("the Hadamard transform is part of the transposing quantiser")
+    torch.manual_seed(7)
+    rows, K, part = 2432, 1024, 1280
+    x = (torch.randn(rows, K, device=DEV) * 2).bfloat16()
+    amax = x.float().abs().max().reshape(1)
+
+    def quantise(t):
+        if transpose:
+            return ext.nvfp4_quantize_transpose(t.t().contiguous(), amax, True, hadamard, 5, 0xB2CD)
+        return ext.nvfp4_quantize(t.contiguous(), amax, True, 5, False)
+
+    q, sf = quantise(x)
+    qp, sfp = quantise(x[:part])
+    assert torch.equal(q[:part], qp) and torch.equal(sf[:sfp.numel()], sfp) and part % 128 == 0
+    if not transpose:
+        assert torch.equal(ext.nvfp4_quantize(x, amax, True, 5, True)[0][:part], ext.nvfp4_quantize(x[:part], amax, True, 5, True)[0])
