@@ -536,8 +536,9 @@ void adamw8_step(Tensor& p, const Tensor& g, Tensor& m8, Tensor& v8, Tensor& ms,
         }
     }
     g_launches += 1;
-    sg::adamw_8bit(p.data_ptr(), p.scalar_type() == at::kFloat, g.data_ptr(), g.scalar_type() == at::kFloat, m8.data_ptr(), v8.data_ptr(), ms.data_ptr(),
-                   vs.data_ptr(), static_cast<const uint8_t*>(opt_ptr(mask)), block_mask, hp.data_ptr<float>(), p.numel(), num_sms(), cur_stream());
+    const char* err = sg::adamw_8bit(p.data_ptr(), p.scalar_type() == at::kFloat, g.data_ptr(), g.scalar_type() == at::kFloat, m8.data_ptr(), v8.data_ptr(), ms.data_ptr(),
+                                     vs.data_ptr(), static_cast<const uint8_t*>(opt_ptr(mask)), block_mask, hp.data_ptr<float>(), p.numel(), num_sms(), cur_stream());
+    TORCH_CHECK(err == nullptr, err ? err : "");
 }
 
 }  // namespace

@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "kernels.h"
+#include "launch_limits.h"
 #include "sm100_ptx.cuh"
 
 namespace sg {
@@ -1239,13 +1240,14 @@ void adamw_fp32(void* p, int p_fp32, const void* g, int g_fp32, float* m, float*
     else if (g_fp32) adamw_fp32_kernel<bf16, float><<<grid, 256, 0, s>>>((bf16*)p, (const float*)g, m, v, mask, hp, n);
     else adamw_fp32_kernel<bf16, bf16><<<grid, 256, 0, s>>>((bf16*)p, (const bf16*)g, m, v, mask, hp, n);
 }
-void adamw_8bit(void* p, int p_fp32, const void* g, int g_fp32, void* m8, void* v8, void* ms, void* vs, const uint8_t* mask, int block_mask,
+const char* adamw_8bit(void* p, int p_fp32, const void* g, int g_fp32, void* m8, void* v8, void* ms, void* vs, const uint8_t* mask, int block_mask,
                 const float* hp, size_t n, int num_sms, cudaStream_t s) {
 #define SG_A8(PT, GT, BM)                                                                                                                       \
     do {                                                                                                                                        \
         constexpr int smem = adam8_stages<PT, GT>() * adam8_slot_bytes<PT, GT>();                                                                 \
         static_assert(3 * (smem + 2048) <= 227 * 1024, "three CTAs per SM");                                                                     \
-        cudaFuncSetAttribute(adamw_8bit_kernel<PT, GT, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   /* of the current device */        \
+        static std::atomic<uint64_t> limit{0};                                                                                                  \
+        if (!raise_smem_limit(reinterpret_cast<const void*>(adamw_8bit_kernel<PT, GT, BM>), smem, limit)) return "raising the shared-memory limit failed (8-bit AdamW)"; \
         const int grid = grid_for(n / 8, ADAM8_THREADS, num_sms, 3);   /* the resident CTAs, each with a full ring */      \
         adamw_8bit_kernel<PT, GT, BM><<<grid, ADAM8_THREADS, smem, s>>>((PT*)p, (const GT*)g, (int8_t*)m8, (uint8_t*)v8, (__half*)ms, (__half*)vs, mask, hp, n); \
     } while (0)
@@ -1255,6 +1257,7 @@ void adamw_8bit(void* p, int p_fp32, const void* g, int g_fp32, void* m8, void* 
         if (p_fp32 && g_fp32) SG_A8(float, float, false); else if (p_fp32) SG_A8(float, bf16, false); else if (g_fp32) SG_A8(bf16, float, false); else SG_A8(bf16, bf16, false);
     }
 #undef SG_A8
+    return cudaGetLastError() == cudaSuccess ? nullptr : "8-bit AdamW launch failed";
 }
 
 }  // namespace sg
