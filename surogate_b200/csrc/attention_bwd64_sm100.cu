@@ -28,6 +28,7 @@
 
 #include "attention_sm100.h"
 #include "gemm_sm100.h"
+#include "launch_limits.h"
 #include "sm100_ptx.cuh"
 
 namespace sg {
@@ -340,15 +341,11 @@ const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const flo
     if ((e = make_tensor_map_2d(&q64, qkv, 2, width, rows, width * 2, 64, 64))) return e;
     if ((e = make_tensor_map_2d(&do128, d_out, 2, owidth, rows, owidth * 2, 64, 128))) return e;
     if ((e = make_tensor_map_2d(&do64, d_out, 2, owidth, rows, owidth * 2, 64, 64))) return e;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(fa_bwd64_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(fa_bwd64_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(fa_bwd64_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(fa_bwd64_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-            return "cudaFuncSetAttribute failed (flash_attn_bwd64)";
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> limit[4];
+    auto raise = [](auto* kernel, std::atomic<uint64_t>& done) { return raise_smem_limit(reinterpret_cast<const void*>(kernel), SMEM, done); };
+    if (!(lo ? raise(fa_bwd64_kernel<true, true>, limit[3]) && raise(fa_bwd64_kernel<false, true>, limit[1])
+             : raise(fa_bwd64_kernel<true, false>, limit[2]) && raise(fa_bwd64_kernel<false, false>, limit[0])))
+        return "raising the shared-memory limit failed (flash_attn_bwd64)";
     if ((lo == nullptr) != (kv_qend == nullptr)) return "flash_attn_bwd: the lower bounds and the per-key-tile query ends come together";
     Params p{static_cast<__nv_bfloat16*>(d_qkv), neg_lse2, delta, T, Hq, Hkv, softmax_scale, softmax_scale * LOG2E, error_flag, prof, lo, kv_qend};
     if (lo) {

@@ -16,6 +16,7 @@
 
 #include "attention_sm100.h"
 #include "gemm_sm100.h"
+#include "launch_limits.h"
 #include "sm100_ptx.cuh"
 
 namespace sg {
@@ -309,13 +310,10 @@ const char* flash_attn_fwd64_sm100(const void* qkv, void* out, float* lse, int B
     if (e) return e;
     e = make_tensor_map_2d(&tm_kv, qkv, 2, width, static_cast<uint64_t>(B) * T, width * 2, 64, 64);
     if (e) return e;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(fa_fwd64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(fa_fwd64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-            return "cudaFuncSetAttribute failed (flash_attn_fwd64)";
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> limit[2];
+    if (!(lo ? raise_smem_limit(reinterpret_cast<const void*>(fa_fwd64_kernel<true>), SMEM_BYTES, limit[1])
+             : raise_smem_limit(reinterpret_cast<const void*>(fa_fwd64_kernel<false>), SMEM_BYTES, limit[0])))
+        return "raising the shared-memory limit failed (flash_attn_fwd64)";
     Params p{static_cast<__nv_bfloat16*>(out), lse, T, Hq, Hkv, softmax_scale * 1.4426950408889634f, error_flag, prof, lo};
     if (lo) fa_fwd64_kernel<true><<<dim3(T / 128, Hq, B), THREADS, SMEM_BYTES, stream>>>(tm_q, tm_kv, p);
     else fa_fwd64_kernel<false><<<dim3(T / 128, Hq, B), THREADS, SMEM_BYTES, stream>>>(tm_q, tm_kv, p);

@@ -12,6 +12,7 @@
 // Replaces the CUTLASS Sm100 block-scaled instantiation of the reference
 // (csrc/src/recipes/nvfp4/kernels/matmul_cutlass_fp4_sm100.cu:41-159).
 #include "gemm_sm100.h"
+#include "launch_limits.h"
 #include "sm100_ptx.cuh"
 
 namespace sg {
@@ -255,12 +256,8 @@ const char* gemm_nvfp4_sm100(const void* a, const void* b, const void* sfa, cons
     if (e) return e;
     e = make_tensor_map_2d(&tmB, b, 1, static_cast<uint64_t>(K) / 2, N, static_cast<uint64_t>(K) / 2, ROW_BYTES, BN);
     if (e) return e;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_nvfp4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-            return "cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed";
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> limit{0};
+    if (!raise_smem_limit(reinterpret_cast<const void*>(gemm_nvfp4_kernel), SMEM_BYTES, limit)) return "raising the shared-memory limit failed (NVFP4 GEMM)";
     Fp4Params p{};
     p.M = M; p.N = N; p.K = K;
     p.sfa = static_cast<const uint8_t*>(sfa);

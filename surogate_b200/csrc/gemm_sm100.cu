@@ -15,6 +15,7 @@
 #include <cuda_fp8.h>
 
 #include "gemm_sm100.h"
+#include "launch_limits.h"
 #include "sm100_ptx.cuh"
 
 namespace sg {
@@ -814,12 +815,8 @@ template <int BN> static const char* launch(const GemmOperand& A, const GemmOper
     if (!p.b_mn) e = make_tensor_map_2d(&tmB, B.ptr, p.elem_bytes, p.K, b_rows, B.row_stride_bytes, BK, BN);
     else e = make_tensor_map_2d(&tmB, B.ptr, p.elem_bytes, p.N, b_rows, B.row_stride_bytes, BK, BK);
     if (e) return e;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess)
-            return "cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed";
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> limit{0};
+    if (!raise_smem_limit(reinterpret_cast<const void*>(gemm_tcgen05_kernel<BN>), C::SMEM_BYTES, limit)) return "raising the shared-memory limit failed (GEMM)";
     int units = p.mode == 0 ? ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) : num_sms;  // grouped: tile count lives on the device
     if (p.splits > 1) units = p.split_from + (units - p.split_from) * p.splits;
     const int grid = units < num_sms ? units : num_sms;
@@ -857,13 +854,10 @@ static const char* launch_pair(const GemmOperand& A, const GemmOperand& B, GemmP
     }
     if (!use_tma_store) tmD = tmA;
     const bool acc = use_tma_store && p.accumulate && !p.out_fp32;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<false>::SMEM_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<true>::SMEM_BYTES) != cudaSuccess)
-            return "cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed (pair GEMM)";
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> limit[2];
+    if (!(acc ? raise_smem_limit(reinterpret_cast<const void*>(gemm_pair_kernel<true>), PairCfg<true>::SMEM_BYTES, limit[1])
+              : raise_smem_limit(reinterpret_cast<const void*>(gemm_pair_kernel<false>), PairCfg<false>::SMEM_BYTES, limit[0])))
+        return "raising the shared-memory limit failed (pair GEMM)";
     const int num_tiles = ((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
     const int units = p.splits > 1 ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
     const int clusters = units < num_sms / 2 ? units : num_sms / 2;

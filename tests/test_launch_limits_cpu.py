@@ -1,8 +1,11 @@
 """Shared-memory limits of the kernels are raised once per device, also when several threads launch first, and a refusal is reported and
 asked for again.  The helper is compiled for the host against a stand-in of the three runtime calls that it makes."""
+import glob
 import os
 import re
 import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "surogate_b200", "csrc")
 
@@ -61,7 +64,9 @@ def test_limits_are_raised_once_per_device(tmp_path):
     assert r.returncode == 0, r.stdout
 
 
-def test_adamw_asks_through_the_helper():
-    """A refused limit would leave the launch, and the update, out without a word."""
-    text = open(os.path.join(CSRC, "kernels.cu")).read()
-    assert not re.search(r"cudaFuncSetAttribute\s*\(", text) and "adamw_8bit_kernel<PT, GT, BM>), smem, limit)) return" in text
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu"))), ids=os.path.basename)
+def test_kernels_ask_through_the_helper(path):
+    """A flag of the whole process, or a call whose result is dropped, leaves the second device of a process without the limit."""
+    text = open(path).read()
+    assert not re.search(r"static\s+bool\s+attr_set", text)
+    assert not re.search(r"cudaFuncSetAttribute\s*\(", text)
