@@ -107,6 +107,23 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& d, bool a_mn, bool b_mn, boo
     TORCH_CHECK(err == nullptr, err ? err : "");
 }
 
+// (CTA pairs, pieces of the cut tiles' contraction, first cut tile, bytes of workspace) with which `gemm` runs such a problem
+std::tuple<bool, int, int, int64_t> gemm_plan(int64_t M, int64_t N, int64_t K, int64_t elem_bytes, bool a_mn, bool b_mn, bool out_fp32, bool accumulate,
+                                              int64_t tile_n, int64_t sm_count) {
+    sg::GemmParams p{};
+    p.M = static_cast<int>(M);
+    p.N = static_cast<int>(N);
+    p.K = static_cast<int>(K);
+    p.elem_bytes = static_cast<int>(elem_bytes);
+    p.a_mn = a_mn;
+    p.b_mn = b_mn;
+    p.out_fp32 = out_fp32;
+    p.accumulate = accumulate;
+    p.tile_n = static_cast<int>(tile_n);
+    const sg::GemmPlan plan = sg::gemm_plan_sm100(p, sm_count > 0 ? static_cast<int>(sm_count) : num_sms());
+    return {plan.pair != 0, plan.splits, plan.split_from, static_cast<int64_t>(4 * (plan.workspace_floats + (plan.splits > 1 ? plan.num_counters : 0)))};
+}
+
 Tensor error_flag_tensor() {
     error_flag_ptr();
     return g_error_flag;
@@ -549,6 +566,8 @@ int* sg_error_flag() { return error_flag_ptr(); }
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("error_flag_tensor", &error_flag_tensor, "the device int32 word kernels set when a bounded wait runs out");
     m.def("gemm", &gemm, "tcgen05 GEMM");
+    m.def("gemm_plan", &gemm_plan, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("elem_bytes") = 2, py::arg("a_mn") = false, py::arg("b_mn") = false,
+          py::arg("out_fp32") = false, py::arg("accumulate") = false, py::arg("tile_n") = 0, py::arg("sm_count") = 0);
     m.def("read_error_flag", &read_error_flag);
     m.def("launch_count", &launch_count, "number of kernels this extension has launched");
     m.def("rmsnorm_fwd", &rmsnorm_fwd);

@@ -14,6 +14,8 @@
 // Replaces the cuBLASLt calls of the reference (csrc/src/kernels/matmul.cpp:447-1000).
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "gemm_sm100.h"
 #include "launch_limits.h"
 #include "sm100_ptx.cuh"
@@ -867,19 +869,22 @@ static const char* launch_pair(const GemmOperand& A, const GemmOperand& B, GemmP
 }
 
 // ------------------------------------------------------------------------------------------------ choice of kernel and split
-// Which kernel runs a dense problem, and into how many pieces the contraction of its last wave of tiles is cut, by estimated time.  The
-// constants are measured (B200, both element widths: a contraction block is 128 bytes deep): one block costs a CTA pair 0.46 us and a
-// single CTA with its 128 x 128 tile 0.36 us; a piece costs its trip through the workspace, its reader all pieces of the tile, and the
-// cleared counters a launch.
+// Which kernel runs a dense problem, and into how many pieces the contraction of its last wave of tiles is cut, by estimated time.  A wave
+// costs its contraction (128-byte blocks) or its epilogue, whichever is longer, and the last one both; a piece costs its trip through the
+// workspace, the warp that adds them every piece; nothing is faster than its operands and output from memory.  The constants are a
+// least-squares fit to 68 000 timings on B200 (11 500 problems, every kernel and split that they allow: profiles/gemm_kernel_choice.md);
+// blocks cost the same in bf16 and FP8.  The estimate is good to 10-20 %, so the count of pair tiles decides (a wave of them: pairs) unless
+// the other kernel is estimated 8 % faster, and a split has to promise 5 %.
 //   pair   : full rate, but 74 tiles of 256 x 256 to a wave.  [1024, 3072] = 16384 deep (48 tiles) in three pieces 164 -> 93 us, [6144, 1024] (96
 //            tiles, the last 22 in three pieces) 204 -> 157 us, [4096, 4096] = 151936 deep in bf16 (256 tiles, 34 in two) 4530 -> 3939 us.
 //   single : four times as many tiles, for small outputs; also the narrow ones (N <= 128), where a pair would multiply padding:
-//            [4096, 16] = 17408 deep 91 -> 45 us in four pieces.
+//            [4096, 16] = 17408 deep 91 -> 45 us in four pieces.  Its fp32 accumulation goes row by row from registers: [64, 151936] += 64
+//            deep takes 94 us, pairs 34 us.
 namespace {
 struct Shape {
-    int tiles, slots;                          // output tiles, tiles that run at once
-    float block_us, piece_us, reader_us;       // per contraction block; per piece of a split tile; per piece for the warp that adds them
-    float split_us;                            // once per split problem
+    int tiles, slots;                               // output tiles, tiles that run at once
+    float fixed_us, block_us, epilogue_us;          // once; per contraction block of a wave; per wave
+    float piece_us, reader_us, split_us;            // per wave of pieces; per piece for the warp that adds them; once per split problem
     int tile_floats;
 };
 struct Split {
@@ -888,15 +893,18 @@ struct Split {
 };
 constexpr int MAX_PIECES = 8;
 constexpr int MIN_PIECE_BLOCKS = 4;
+constexpr float SPLIT_GAIN = 0.95f, KERNEL_GAIN = 0.92f;
+constexpr float STREAM_BYTES_PER_US = 4.0e6f;
 
-Split best_split(const Shape& h, int num_k) {
-    const int rest = h.tiles % h.slots;
-    const float full = static_cast<float>(h.tiles / h.slots) * num_k * h.block_us;
-    Split best{full + (rest ? num_k * h.block_us : 0.f), h.tiles, 1};
+Split best_split(const Shape& h, int num_k, float stream_us) {
+    const int full = h.tiles / h.slots, rest = h.tiles % h.slots;
+    const float k_us = num_k * h.block_us, wave_us = std::max(k_us, h.epilogue_us);
+    const int waves = full + (rest ? 1 : 0);
+    Split best{std::max(stream_us, h.fixed_us + (waves - 1) * wave_us + k_us + h.epilogue_us), h.tiles, 1};
     for (int s = 2; rest && s <= MAX_PIECES && num_k / s >= MIN_PIECE_BLOCKS && rest * s <= 3 * h.slots; ++s) {
-        const int waves = (rest * s + h.slots - 1) / h.slots;
-        const float us = full + waves * (((num_k + s - 1) / s) * h.block_us + h.piece_us) + s * h.reader_us + h.split_us;
-        if (us < best.us * 0.97f) best = Split{us, h.tiles - rest, s};
+        const int piece_waves = (rest * s + h.slots - 1) / h.slots;
+        const float us = h.fixed_us + full * wave_us + piece_waves * (((num_k + s - 1) / s) * h.block_us + h.piece_us) + s * h.reader_us + h.split_us + h.epilogue_us;
+        if (std::max(stream_us, us) < best.us * SPLIT_GAIN) best = Split{std::max(stream_us, us), h.tiles - rest, s};
     }
     return best;
 }
@@ -905,12 +913,18 @@ Split best_split(const Shape& h, int num_k) {
 GemmPlan gemm_plan_sm100(const GemmParams& p, int num_sms) {
     GemmPlan plan{0, 1, 0, 0, 0};
     if (p.mode != 0 || p.M <= 0 || p.N <= 0 || p.K <= 0) return plan;
-    const int num_k = (p.K * p.elem_bytes + TILE_K_BYTES - 1) / TILE_K_BYTES;
+    const int num_k = static_cast<int>((static_cast<long long>(p.K) * p.elem_bytes + TILE_K_BYTES - 1) / TILE_K_BYTES);
     auto up = [](int a, int b) { return (a + b - 1) / b; };
-    const Shape pair{up(p.M, PAIR_BM) * up(p.N, PAIR_BN), num_sms / 2, 0.46f, 3.0f, 2.5f, 5.0f, PAIR_BM * PAIR_BN};
-    const Shape single{up(p.M, BM) * up(p.N, 128), num_sms, 0.36f, 1.5f, 1.2f, 4.0f, BM * 128};
-    const Split sp = best_split(pair, num_k), ss = best_split(single, num_k);
-    int use_pair = p.tile_n == 512 || (p.tile_n == 0 && p.N > 128 && p.M > 128 && sp.us <= ss.us);
+    const int out = (p.out_fp32 ? 2 : 0) + (p.accumulate ? 1 : 0), mn = (p.a_mn ? 1 : 0) + (p.b_mn ? 1 : 0);   // bf16, bf16 +=, fp32, fp32 +=
+    constexpr float pair_out[4] = {4.0f, 5.4f, 5.2f, 5.8f}, single_out[4] = {3.7f, 7.7f, 5.3f, 13.0f}, single_block[3] = {0.26f, 0.27f, 0.32f};
+    const Shape pair{up(p.M, PAIR_BM) * up(p.N, PAIR_BN), num_sms / 2, 1.6f, 0.41f, pair_out[out], 7.2f, 1.2f, 1.5f, PAIR_BM * PAIR_BN};
+    const float single_piece = p.M < 16 ? 10.3f : 6.3f;        // boxes with fewer than 16 rows inside A arrive slowly: 2-4 us more per piece
+    const Shape single{up(p.M, BM) * up(p.N, 128), num_sms, 0.4f, single_block[mn], single_out[out], single_piece, 0.4f, 0.4f, BM * 128};
+    const float stream_us = (static_cast<float>(p.elem_bytes) * p.K * (static_cast<float>(p.M) + p.N) +
+                             (p.out_fp32 ? 4.f : 2.f) * (p.accumulate ? 2.f : 1.f) * p.M * p.N) / STREAM_BYTES_PER_US;
+    const Split sp = best_split(pair, num_k, stream_us), ss = best_split(single, num_k, stream_us);
+    int use_pair = p.N > 128 && (pair.tiles >= pair.slots ? !(ss.us < KERNEL_GAIN * sp.us) : sp.us < KERNEL_GAIN * ss.us);
+    if (p.tile_n != 0) use_pair = p.tile_n == 512;
     plan.pair = use_pair;
     if (p.tile_n == 256 || p.tile_n == 128) return plan;        // forced single-CTA tiles: never split
     const Split& c = use_pair ? sp : ss;
