@@ -98,9 +98,12 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& d, bool a_mn, bool b_mn, boo
     const sg::GemmPlan plan = sg::gemm_plan_sm100(p, num_sms());
     Tensor ws;
     if (plan.splits > 1) {
-        ws = torch::empty({static_cast<int64_t>(plan.workspace_floats + plan.num_counters)}, d.options().dtype(at::kFloat));
-        p.workspace = ws.data_ptr<float>();
-        p.counters = reinterpret_cast<int*>(p.workspace + plan.workspace_floats);
+        try {
+            ws = torch::empty({static_cast<int64_t>(plan.workspace_floats + plan.num_counters)}, d.options().dtype(at::kFloat));
+            p.workspace = ws.data_ptr<float>();
+            p.counters = reinterpret_cast<int*>(p.workspace + plan.workspace_floats);
+        } catch (const c10::OutOfMemoryError&) {      // a full device: the same kernel, unsplit, needs no memory
+        }
     }
     g_launches += 1;
     const char* err = sg::gemm_sm100(A, B, p, num_sms(), cur_stream());

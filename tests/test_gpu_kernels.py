@@ -139,6 +139,30 @@ def test_gemm_with_a_split_contraction(ext, M, N, K, tile_n, a_mn, b_mn, fp8):
     assert _rel_err(acc32, D0 + 0.5 * ref) < 2e-5
 
 
+def test_gemm_runs_unsplit_when_the_workspace_does_not_fit(ext):
+    """A split contraction takes up to 58 MB of workspace; a device with less to spare still multiplies.  (The allocator is limited, not the
+    device filled.)"""
+    from surogate_b200.runtime.ops_cuda import gemm
+
+    torch.manual_seed(0)
+    M, N, K = 1024, 3072, 16384
+    a, b = torch.randn(K, M, device=DEV).bfloat16(), torch.randn(K, N, device=DEV).bfloat16()
+    assert ext.gemm_plan(M, N, K, 2, True, True, False, False, 0, 148)[3] > 20 << 20
+    want, out = gemm(a, b, a_mn=True, b_mn=True), torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    ref = a.float().t() @ b.float()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) / total)
+        gemm(a, b, out, a_mn=True, b_mn=True)
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    _check_flag()
+    assert _rel_err(out, ref) < 2.5e-3 and _rel_err(want, ref) < 2.5e-3
+
+
 def test_gemm_bf16_accumulation_with_a_short_contraction(ext):
     """D += A.B^T where D is the traffic (adapter updates, gradient accumulation): its tiles travel through shared memory both ways."""
     from surogate_b200.runtime.ops_cuda import gemm
