@@ -97,16 +97,18 @@ def test_gemm_cta_pair(ext, M, N, K, a_mn, b_mn, fp8):
     _check_flag()
 
 
-SPLIT_SHAPES = [(16, 5120, 4096, 0), (1024, 16, 8192, 0), (136, 200, 2056, 0),     # single CTAs, every tile cut
-                (1024, 1024, 6144, 512), (3000, 1000, 4104, 0),                     # CTA pairs, every tile cut, ragged edges
-                (2560, 2048, 2112, 512), (5376, 1032, 1536, 512)]                   # whole waves, then cut tiles
+# M, N, K, tile_n, whole tiles before the cut ones
+SPLIT_SHAPES = [(16, 5120, 16384, 0, False), (1024, 16, 16384, 0, False), (136, 200, 16400, 0, False),      # single CTAs, every tile cut
+                (640, 4104, 16400, 0, True),                                                                # single CTAs, a wave of whole tiles first
+                (1024, 1024, 16384, 512, False), (2000, 1000, 16400, 512, False),                           # CTA pairs, every tile cut, ragged edges
+                (2560, 2048, 8192, 512, True), (5376, 1032, 16400, 512, True), (5000, 2056, 16400, 0, True)]  # CTA pairs, whole waves first
 
 
-@pytest.mark.parametrize("M,N,K,tile_n", SPLIT_SHAPES)
+@pytest.mark.parametrize("M,N,K,tile_n,whole", SPLIT_SHAPES)
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("fp8", [False, True])
-def test_gemm_with_a_split_contraction(ext, M, N, K, tile_n, a_mn, b_mn, fp8):
-    """Shapes whose tiles leave SMs idle are cut along the contraction.  bf16 and fp32 outputs, plain and accumulated, against fp32
+def test_gemm_with_a_split_contraction(ext, M, N, K, tile_n, whole, a_mn, b_mn, fp8):
+    """Shapes whose tiles leave SMs idle are cut along the contraction (the plan is asked, so that other constants cannot empty this test).  bf16 and fp32 outputs, plain and accumulated, against fp32
     PyTorch: the error is the rounding of the output (2^-9 per element, twice with accumulation) and of fp32 sums; and the same bits twice,
     since the pieces are added in a fixed order."""
     from surogate_b200.runtime.ops_cuda import gemm
@@ -114,6 +116,9 @@ def test_gemm_with_a_split_contraction(ext, M, N, K, tile_n, a_mn, b_mn, fp8):
     es = 1 if fp8 else 2
     if (a_mn and M * es % 16) or (b_mn and N * es % 16) or K * es % 16:
         pytest.skip("row stride must be a multiple of 16 bytes")
+    for out_fp32, accumulate in ((False, False), (False, True), (True, True)):
+        pair, pieces, first_cut, _ = ext.gemm_plan(M, N, K, es, a_mn, b_mn, out_fp32, accumulate, tile_n, 148)
+        assert pieces > 1 and (first_cut > 0) == whole and (pair or tile_n != 512)
     torch.manual_seed(M + N + K)
     dt = torch.float8_e4m3fn if fp8 else torch.bfloat16
     a = torch.randn(*((K, M) if a_mn else (M, K)), device=DEV).to(dt)
@@ -292,7 +297,7 @@ def test_rmsnorm_forward_widths(ext, rows, C):
 
 @pytest.mark.parametrize("rows,M", [(1, 8), (3, 264), (2, 12288), (8193, 768), (1025, 2056)])
 def test_swiglu_row_counts(ext, rows, M):
-    """Row counts that leave the second row of a thread's pair behind the end, and one row."""
+    """One row, row counts off the grid's stride, and widths of one to many vectors."""
     torch.manual_seed(rows + M)
     x, dy = torch.randn(rows, 2 * M, device=DEV).bfloat16(), torch.randn(rows, M, device=DEV).bfloat16()
     xr = x.float().requires_grad_(True)
@@ -385,7 +390,8 @@ def test_embedding_gradient_of_narrow_rows_needs_no_copy_of_the_table(ext, C, sh
 @pytest.mark.parametrize("n", [8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 24, 3 * 148 * 8 * 256 * 8 + 8])
 @pytest.mark.parametrize("e5m2", [False, True])
 def test_quantize_fp8_counts(ext, n, e5m2):
-    """Counts at which a thread has no, one, some or all of its four vectors: the bits of PyTorch's conversion (saturating), and the abs-max."""
+    """Counts of one vector, one block, one whole trip of the grid (148 SMs x 8 blocks x 256 threads x 8 values), a few vectors more, and
+    several trips: the bits of PyTorch's conversion (saturating), and the abs-max."""
     torch.manual_seed(n % 1000)
     x = (torch.randn(n, device=DEV) * 200).bfloat16()
     x[-1] = -3000.0
@@ -781,6 +787,50 @@ def test_moe_zero_rows(ext, E, cap, C, pads):
         for e in range(E):
             want[int(offsets[e] + counts[e]):int(offsets[e + 1])] = 0
     assert torch.equal(buf.float().cpu(), want)
+
+
+def test_moe_buffers_start_unwritten(ext):
+    """The expert buffers of a training step are not cleared as a whole: every row is written by the permutation, the grouped GEMM, the
+    un-permutation's backward or the clear of the rows without a token.  With NaN in all of them beforehand (and in the block that the
+    allocator hands out again), no NaN is left, rows without a token are zero, and the weight gradient, which contracts over them, is right."""
+    torch.manual_seed(1)
+    tokens, C, E, K, Nout = 500, 256, 16, 4, 384
+    nan = float("nan")
+    x = torch.randn(tokens, C, device=DEV).bfloat16()
+    ti = torch.stack([torch.randperm(E - 1, device=DEV)[:K] for _ in range(tokens)]).to(torch.int32)      # the last expert gets nothing
+    counts = torch.bincount(ti.reshape(-1).long(), minlength=E).to(torch.int32)
+    cap = tokens * K + E * 128
+    offsets, cursors = torch.empty(E + 1, dtype=torch.int32, device=DEV), torch.empty(E, dtype=torch.int32, device=DEV)
+    err = ext.error_flag_tensor()
+    ext.moe_offsets(counts, offsets, cursors, cap, err)
+    xp = torch.full((cap, C), nan, dtype=torch.bfloat16, device=DEV)
+    ext.moe_zero_rows(xp, offsets, counts)
+    row_map = torch.empty(tokens * K, dtype=torch.int32, device=DEV)
+    ext.moe_permute(x, ti, offsets, cursors, row_map, xp, 0, E)
+    empty = torch.ones(cap, dtype=torch.bool, device=DEV)
+    empty[row_map.long()] = False
+    assert not xp[empty].any() and torch.equal(xp[row_map.long()], x.repeat_interleave(K, 0))
+    w = torch.randn(E, Nout, C, device=DEV).bfloat16() * 0.1
+    y = torch.full((cap, Nout), nan, dtype=torch.bfloat16, device=DEV)
+    ext.moe_zero_rows(y, offsets)
+    ext.gemm_grouped(xp, w, y, offsets, 1, False, False, 1.0, None, None, err)
+    ref_y = torch.einsum("rc,rnc->rn", x.repeat_interleave(K, 0).float(), w[ti.reshape(-1).long()].float())
+    assert not y[empty].any() and _rel_err(y[row_map.long()], ref_y) < 6e-3
+    tw, dout = torch.rand(tokens, K, device=DEV), torch.randn(tokens, Nout, device=DEV).bfloat16()
+    torch.full((cap, Nout), nan, dtype=torch.bfloat16, device=DEV)           # freed at once
+    d_yp, d_tw = ext.moe_unpermute_bwd(dout, y, tw, row_map, offsets, counts)
+    want_d, want_w = ext.moe_unpermute_bwd(dout, y, tw, row_map)
+    assert torch.equal(d_yp, want_d) and torch.equal(d_tw, want_w) and not d_yp[empty].any()
+    dx = torch.full((cap, C), nan, dtype=torch.bfloat16, device=DEV)
+    ext.moe_zero_rows(dx, offsets)
+    ext.gemm_grouped(d_yp, w, dx, offsets, 1, True, False, 1.0, None, None, err)
+    assert not dx[empty].any() and not dx.isnan().any()
+    dw = torch.zeros(E, Nout, C, dtype=torch.float32, device=DEV)
+    ext.gemm_grouped(d_yp, xp, dw, offsets, 2, True, True, 1.0, None, None, err)
+    ref_dw = torch.zeros_like(dw)
+    ref_dw.index_add_(0, ti.reshape(-1).long(), torch.einsum("rn,rc->rnc", d_yp[row_map.long()].float(), x.repeat_interleave(K, 0).float()))
+    assert _rel_err(dw, ref_dw) < 6e-3
+    _check_flag()
 
 
 def test_embedding_rejects_out_of_range_token_ids():
