@@ -5,8 +5,8 @@
 //   dK/dV pass: resident (K, V) of one 128-key tile of one KV head, streamed (Q, dO) tiles of the G query heads that share it:
 //               X = S^T, Y = dP^T, P^T = exp2(S^T - lse), dS^T = P^T o (dP^T - delta) scale; dV += P^T dO, dK += dS^T Q.
 //   dQ pass   : resident (Q, dO) of one 128-query tile, streamed (K, V) tiles: X = S, Y = dP, dS = P o (dP - delta) scale; dQ += dS K.
-// dS is scaled before it is rounded to bf16: scaling the finished dK / dQ instead saved nothing (the softmax warps wait for the tensor pipe) and
-// its error against fp64 was 0.2-0.8 % larger over four shapes.
+// dS is scaled before it is rounded to bf16, at no cost: delta comes times -scale, so that the difference and the scale are one fused
+// multiply-add.  Scaling the finished dK / dQ instead had an error against fp64 that was 0.2-0.8 % larger over four shapes.
 //
 // Two groups of four softmax warps take alternate items.  Each group has its own pair of score accumulators (X, Y) in TMEM, reads them,
 // and writes P and dS as bf16 over them, from where the accumulating MMAs take their A operand: no copy in shared memory, no proxy
@@ -45,7 +45,7 @@ constexpr float LOG2E = 1.4426950408889634f;
 struct Params {
     __nv_bfloat16* d_qkv;
     const float* neg_lse2;   // [B, Hq, T]: -lse * log2(e)
-    const float* delta;      // [B, Hq, T]
+    const float* neg_delta;  // [B, Hq, T]: -delta * scale
     int T, Hq, Hkv;
     float scale, scale_log2;
     int* error_flag;
@@ -98,7 +98,7 @@ __device__ __forceinline__ void mma_acc_k64(uint32_t d_tmem, uint32_t a_tmem, ui
 }
 
 // ------------------------------------------------------------------------------------------------ the kernel
-// R1 | R2 | ring (S1, S2) x 4 | barriers | row statistics of the ring's query tiles (dK/dV pass): 64 x -lse2, delta, lo
+// R1 | R2 | ring (S1, S2) x 4 | barriers | row statistics of the ring's query tiles (dK/dV pass): 64 x -lse2, -delta, lo
 constexpr int RING = 4;
 constexpr int OFF_R2 = T128, OFF_RING = 2 * T128, STAGE = 2 * T64, OFF_BAR = OFF_RING + RING * STAGE, OFF_VEC = OFF_BAR + 256;
 constexpr int VEC = 3 * 64 * 4;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
                     const size_t stat = (static_cast<size_t>(b) * p.Hq + h) * p.T + q0;
                     const uint32_t dv = s_vec + st * VEC;
                     bulk_load(dv, p.neg_lse2 + stat, 256, bar(B_RFULL + st));
-                    bulk_load(dv + 256, p.delta + stat, 256, bar(B_RFULL + st));
+                    bulk_load(dv + 256, p.neg_delta + stat, 256, bar(B_RFULL + st));
                     if (HAS_LO) bulk_load(dv + 512, p.lo + qr, 256, bar(B_RFULL + st));
                     tma_load_2d(d1, &tm_qkv64, h * D, qr, bar(B_RFULL + st));
                     tma_load_2d(d1 + H64, &tm_qkv64, h * D + 64, qr, bar(B_RFULL + st));
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
         if (IS_DQ) {
             const size_t idx = (static_cast<size_t>(b) * p.Hq + head) * p.T + row_abs;
             row_neg_lse2 = p.neg_lse2[idx];
-            row_dl = p.delta[idx];
+            row_dl = p.neg_delta[idx];
             if (HAS_LO) row_lo = __ldg(p.lo + row0 + row_abs);
         }
         const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), ds_scale2 = make_float2(p.scale, p.scale);
@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
                     for (int k = 0; k < 4; k += 2) {
                         const float2 e = fma2(make_float2(__uint_as_float(x[c + k]), __uint_as_float(x[c + k + 1])), scale2, k ? make_float2(nl.z, nl.w) : make_float2(nl.x, nl.y));
                         const float2 pr = make_float2(ex2_approx(e.x), ex2_approx(e.y));
-                        const float2 nd = k ? make_float2(-d4.z, -d4.w) : make_float2(-d4.x, -d4.y);
-                        const float2 ds = mul2(mul2(pr, add2(make_float2(__uint_as_float(y[c + k]), __uint_as_float(y[c + k + 1])), nd)), ds_scale2);
+                        const float2 nd = k ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
+                        const float2 ds = mul2(pr, fma2(make_float2(__uint_as_float(y[c + k]), __uint_as_float(y[c + k + 1])), ds_scale2, nd));
                         const __nv_bfloat162 hp = __floats2bfloat162_rn(pr.x, pr.y), hs = __floats2bfloat162_rn(ds.x, ds.y);
                         if (!IS_DQ) pb[hf * 16 + (c + k) / 2] = reinterpret_cast<const uint32_t&>(hp);
                         sb[hf * 16 + (c + k) / 2] = reinterpret_cast<const uint32_t&>(hs);
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(THREADS, 1) fa_bwd64_kernel(const __grid_const
 
 }  // namespace fb64
 
-const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const float* neg_lse2, const float* delta, void* d_qkv, int B, int T, int Hq, int Hkv,
+const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const float* neg_lse2, const float* neg_delta, void* d_qkv, int B, int T, int Hq, int Hkv,
                                    float softmax_scale, int* error_flag, cudaStream_t stream, long long* prof, const int* lo, const int* kv_qend) {
     using namespace fb64;
     if (T % 128 != 0) return "flash_attn_bwd: T must be a multiple of 128";
@@ -347,7 +347,7 @@ const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const flo
              : raise(fa_bwd64_kernel<true, false>, limit[2]) && raise(fa_bwd64_kernel<false, false>, limit[0])))
         return "raising the shared-memory limit failed (flash_attn_bwd64)";
     if ((lo == nullptr) != (kv_qend == nullptr)) return "flash_attn_bwd: the lower bounds and the per-key-tile query ends come together";
-    Params p{static_cast<__nv_bfloat16*>(d_qkv), neg_lse2, delta, T, Hq, Hkv, softmax_scale, softmax_scale * LOG2E, error_flag, prof, lo, kv_qend};
+    Params p{static_cast<__nv_bfloat16*>(d_qkv), neg_lse2, neg_delta, T, Hq, Hkv, softmax_scale, softmax_scale * LOG2E, error_flag, prof, lo, kv_qend};
     if (lo) {
         fa_bwd64_kernel<false, true><<<dim3(T / 128, Hkv, B), THREADS, SMEM, stream>>>(q128, q64, do128, do64, p);
         fa_bwd64_kernel<true, true><<<dim3(T / 128, Hq, B), THREADS, SMEM, stream>>>(q128, q64, do128, do64, p);
@@ -358,10 +358,11 @@ const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const flo
     return cudaGetLastError() == cudaSuccess ? nullptr : "flash_attn_bwd64 launch failed";
 }
 
-// Row statistics of the backward in the layout it reads, [B, Hq, T]: delta = sum_d dO * O and -lse * log2(e).  Half a warp per (token, head);
+// Row statistics of the backward in the layout it reads, [B, Hq, T]: -scale * sum_d dO * O and -lse * log2(e).  Half a warp per (token, head);
 // a block takes 16 consecutive tokens of one head, so its results are two whole sectors.
 __global__ void __launch_bounds__(256) fa_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse,
-                                                       float* __restrict__ neg_lse2, float* __restrict__ delta, int T, int Hq, unsigned blocks) {
+                                                       float* __restrict__ neg_lse2, float* __restrict__ neg_delta, int T, int Hq, float scale,
+                                                       unsigned blocks) {
     const int sub = threadIdx.x & 15;
     for (unsigned blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
         const unsigned h = blk % Hq;
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(256) fa_delta_kernel(const __nv_bfloat16* __re
         for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
         if (sub == 0) {
             const size_t dst = (tok / T * Hq + h) * T + tok % T;
-            delta[dst] = s;
+            neg_delta[dst] = -s * scale;
             neg_lse2[dst] = -lse[it] * fb64::LOG2E;
         }
     }
@@ -393,10 +394,10 @@ const char* flash_attn_bwd_sm100(const void* qkv, const void* out, const void* d
     const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(B) * T / 16 * Hq);
     if (blocks == 0) return nullptr;
     const unsigned cap = static_cast<unsigned>(num_sms) * 32;
-    float* delta = stats + static_cast<size_t>(B) * T * Hq;
-    fa_delta_kernel<<<blocks < cap ? blocks : cap, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), lse, stats, delta,
-                                                                      T, Hq, blocks);
-    return flash_attn_bwd64_sm100(qkv, d_out, stats, delta, d_qkv, B, T, Hq, Hkv, softmax_scale, error_flag, stream, prof, lo, kv_qend);
+    float* neg_delta = stats + static_cast<size_t>(B) * T * Hq;
+    fa_delta_kernel<<<blocks < cap ? blocks : cap, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), lse, stats,
+                                                                      neg_delta, T, Hq, softmax_scale, blocks);
+    return flash_attn_bwd64_sm100(qkv, d_out, stats, neg_delta, d_qkv, B, T, Hq, Hkv, softmax_scale, error_flag, stream, prof, lo, kv_qend);
 }
 
 }  // namespace sg

@@ -17,8 +17,8 @@ const char* flash_attn_bwd_sm100(const void* qkv, const void* out, const void* d
                                  int Hkv, float softmax_scale, int* error_flag, int num_sms, cudaStream_t stream, const int* lo = nullptr,
                                  const int* kv_qend = nullptr, long long* prof = nullptr);
 
-// The two backward kernels alone; neg_lse2 = -lse * log2(e) and delta are [B, Hq, T].
-const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const float* neg_lse2, const float* delta, void* d_qkv, int B, int T, int Hq, int Hkv,
+// The two backward kernels alone; neg_lse2 = -lse * log2(e) and neg_delta = -softmax_scale * delta are [B, Hq, T].
+const char* flash_attn_bwd64_sm100(const void* qkv, const void* d_out, const float* neg_lse2, const float* neg_delta, void* d_qkv, int B, int T, int Hq, int Hkv,
                                    float softmax_scale, int* error_flag, cudaStream_t stream, long long* prof = nullptr, const int* lo = nullptr,
                                    const int* kv_qend = nullptr);
 
