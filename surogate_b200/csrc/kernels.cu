@@ -359,21 +359,22 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict_
 // ------------------------------------------------------------------------------------------ QK-norm + RoPE
 // Half a warp per (token, head); head_dim 128: lane s = lane & 15 of the half holds elements [8s, 8s+8) (one 16-byte access), the
 // rotary partner (i +/- 64) lives in lane s ^ 8 of the same half.  A warp works on one token at a time and walks all of its heads,
-// two at a time (one per half-warp).  A block takes eight tokens at a time (forward: four, two warps to a token); its threads evaluate the
-// sines and cosines of all of them together, each angle once, into shared memory (two tables in turn, so one barrier per group of tokens).
-// Evaluated in every lane that uses them they cost four times the work and the registers of a third resident block.  Eight tokens to a
-// block of the forward left a second wave of few blocks at 4096 tokens.  On B200, in L2, with angles per lane -> eight tokens -> four,
+// two at a time (one per half-warp).  A block takes TOK tokens at a time; its threads evaluate the sines and cosines of all of them
+// together, each angle once, into shared memory (two tables in turn, so one barrier per group of tokens).  Evaluated in every lane that
+// uses them they cost four times the work and the registers of a third resident block.  TOK is eight (a warp to a token), or four (two) in the
+// forward from 17 heads on, where eight left a second wave of few blocks at 4096 tokens; up to 16 heads the second warp would have half a
+// batch of loads or none (1 x 333 x 32 heads 8.6 -> 5.6 us with four, 2 x 1024 x 7 heads 4.9 -> 8.0).  On B200, in L2, with angles per lane -> eight tokens -> four,
 // 2 x 2048 x 48 heads 31.3 -> 33.1 -> 30.3 us,
 // 2 x 4096 x 48 61.8 -> 53.7 -> 54.2, 1 x 1000 x 32 8.5 -> 8.6 -> 7.0; backward (eight) 95.3 -> 93.0 us at 2 x 4096 x 48.
 // Layout per token: [Hq heads | Hkv heads (K) | Hkv heads (V)] x D.  V heads are copied (forward) / passed through (backward).
 constexpr int ROPE_PAIRS_IN_FLIGHT = 4;      // head pairs whose loads are issued before the first is used
-constexpr int rope_tokens(bool backward) { return backward ? 8 : 4; }
+constexpr int ROPE_SPLIT_HEADS = 2 * 2 * ROPE_PAIRS_IN_FLIGHT;      // more heads than two batches of loads: two warps to a token
 __device__ __forceinline__ float half_warp_sum(float v) {
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-template <bool BACKWARD>
+template <bool BACKWARD, int TOK>
 __global__ void __launch_bounds__(256, BACKWARD ? 2 : 3) qk_norm_rope_kernel(const bf16* __restrict__ in, const bf16* __restrict__ qkv_pre, const bf16* __restrict__ qw,
                                                            const bf16* __restrict__ kw, const int* __restrict__ pos, bf16* __restrict__ out,
                                                            float* __restrict__ q_rstd, float* __restrict__ k_rstd, float* __restrict__ dqw,
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(256, BACKWARD ? 2 : 3) qk_norm_rope_kernel(con
     constexpr int D = 128;
     constexpr int U = ROPE_PAIRS_IN_FLIGHT;
     __shared__ float sdw[2][D];
-    constexpr int TOK = rope_tokens(BACKWARD), WPT = 8 / TOK;     // tokens of a block, warps per token
+    constexpr int WPT = 8 / TOK;     // warps per token
     __shared__ alignas(16) float trig[2][TOK][2][D / 2];   // [table][token][cos | sin][frequency]
     const bool multi_axis = (lim_h | lim_w) != 0;
     if (BACKWARD) {
@@ -1173,14 +1174,18 @@ void zero_empty_groups(void* out, const int* offsets, int groups, size_t bytes_p
 }
 void qk_norm_rope_fwd(const void* qkv, const void* qw, const void* kw, const int* pos, void* out, float* q_rstd, float* k_rstd, size_t tokens, int Hq,
                       int Hkv, float eps, float theta, int lim_h, int lim_w, int num_sms, cudaStream_t s) {
-    qk_norm_rope_kernel<false><<<grid_for(tokens, rope_tokens(false), num_sms, 16), 256, 0, s>>>((const bf16*)qkv, nullptr, (const bf16*)qw, (const bf16*)kw, pos,
-                                                                                   (bf16*)out, q_rstd, k_rstd, nullptr, nullptr, tokens, Hq, Hkv, eps,
-                                                                                   log2f(theta), lim_h, lim_w);
+#define SG_QR(TOK)                                                                                                                               \
+    qk_norm_rope_kernel<false, TOK><<<grid_for(tokens, TOK, num_sms, 64 / TOK), 256, 0, s>>>((const bf16*)qkv, nullptr, (const bf16*)qw, (const bf16*)kw, \
+                                                                                             pos, (bf16*)out, q_rstd, k_rstd, nullptr, nullptr, tokens, \
+                                                                                             Hq, Hkv, eps, log2f(theta), lim_h, lim_w)
+    if (Hq + 2 * Hkv > ROPE_SPLIT_HEADS) SG_QR(4);
+    else SG_QR(8);
+#undef SG_QR
 }
 void qk_norm_rope_bwd(const void* d_out, const void* qkv_pre, const void* qw, const void* kw, const int* pos, void* d_qkv, float* q_rstd,
                       float* k_rstd, float* dqw, float* dkw, size_t tokens, int Hq, int Hkv, float eps, float theta, int lim_h, int lim_w, int num_sms,
                       cudaStream_t s) {
-    qk_norm_rope_kernel<true><<<grid_for(tokens, rope_tokens(true), num_sms, 4), 256, 0, s>>>((const bf16*)d_out, (const bf16*)qkv_pre, (const bf16*)qw,
+    qk_norm_rope_kernel<true, 8><<<grid_for(tokens, 8, num_sms, 4), 256, 0, s>>>((const bf16*)d_out, (const bf16*)qkv_pre, (const bf16*)qw,
                                                                                      (const bf16*)kw, pos, (bf16*)d_qkv, q_rstd, k_rstd, dqw, dkw, tokens,
                                                                                      Hq, Hkv, eps, log2f(theta), lim_h, lim_w);
 }

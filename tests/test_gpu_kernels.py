@@ -447,6 +447,28 @@ def test_qk_norm_rope(ext, B, T, Hq, Hkv):
     assert _rel_err(out2, r2) < 5e-3
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (5, 1), (8, 4), (9, 4), (16, 1), (13, 6), (32, 8)])
+@pytest.mark.parametrize("tokens", [1, 4, 5, 13])
+def test_qk_norm_rope_forward_head_counts(ext, Hq, Hkv, tokens):
+    """Up to 16 heads a warp takes a token, from 17 on two warps share it (3, 7, 16, 17, 18, 25 and 48 here), with token counts around a block's four
+    and eight: fp64 on the same bf16 inputs, one bf16 rounding."""
+    torch.manual_seed(Hq * tokens)
+    H, Dh = Hq + 2 * Hkv, 128
+    qkv = torch.randn(1, tokens, H * Dh, device=DEV).bfloat16()
+    qw, kw = (1 + 0.1 * torch.randn(Dh, device=DEV)).bfloat16(), (1 + 0.1 * torch.randn(Dh, device=DEV)).bfloat16()
+    pos = torch.randint(0, 500, (1, tokens), device=DEV, dtype=torch.int32)
+    out, q_rstd, k_rstd = ext.qk_norm_rope_fwd(qkv, qw, kw, pos, Hq, Hkv, Dh, 1e-6, 1e4)
+    x = qkv.double().view(tokens, H, Dh)
+    rstd = torch.rsqrt(x.pow(2).mean(-1) + 1e-6)
+    n = x * rstd[..., None] * torch.cat([qw.double().expand(Hq, Dh), kw.double().expand(Hkv, Dh), torch.ones(Hkv, Dh, device=DEV, dtype=torch.double)])
+    ang = pos[0].double()[:, None, None] * 1e4 ** (-torch.arange(64, device=DEV).double() / 64)
+    rot = torch.cat([n[..., :64] * ang.cos() - n[..., 64:] * ang.sin(), n[..., 64:] * ang.cos() + n[..., :64] * ang.sin()], -1)
+    got = out.view(tokens, H, Dh)
+    assert torch.equal(got[:, Hq + Hkv:], qkv.view(tokens, H, Dh)[:, Hq + Hkv:])
+    assert _rel_err(got[:, :Hq + Hkv], rot[:, :Hq + Hkv].float()) < 3e-3
+    assert torch.allclose(q_rstd.view(tokens, Hq).double(), rstd[:, :Hq], rtol=1e-5) and torch.allclose(k_rstd.view(tokens, Hkv).double(), rstd[:, Hq:Hq + Hkv], rtol=1e-5)
+
+
 def test_qk_norm_rope_multi_axis_positions(ext):
     """(t, h, w) rotary positions: frequency j reads the height row if j % 3 == 1 and j < 3 * sec_h, the width row if
     j % 3 == 2 and j < 3 * sec_w, else the temporal row; forward and backward against the PyTorch op."""
