@@ -603,52 +603,54 @@ __global__ void __launch_bounds__(EMB_COLS / VEC) embedding_bwd_sorted_kernel(co
     const int i = blockIdx.x;
     const int id = sorted_ids[i];
     if (id < 0 || id >= V || (i > 0 && sorted_ids[i - 1] == id)) return;
-    const int c = blockIdx.y * EMB_COLS + threadIdx.x * VEC;
-    if (c >= C) return;
     using Word = typename EmbWord<VEC>::T;
-    float acc[VEC];
+    for (int c = blockIdx.y * EMB_COLS + threadIdx.x * VEC; c < C; c += gridDim.y * EMB_COLS) {
+        float acc[VEC];
 #pragma unroll
-    for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
-    for (int j = i;; j += EMB_AHEAD) {
-        bool mine[EMB_AHEAD];
-        long long src[EMB_AHEAD];
+        for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
+        if (i + 1 == n || sorted_ids[i + 1] != id) {      // most ids of a batch without frequent ones
+            emb_unpack(*reinterpret_cast<const Word*>(d_out + static_cast<size_t>(order[i]) * C + c), acc);
+        } else for (int j = i;; j += EMB_AHEAD) {
+            bool mine[EMB_AHEAD];
+            long long src[EMB_AHEAD];
 #pragma unroll
-        for (int u = 0; u < EMB_AHEAD; ++u) {
-            mine[u] = j + u < n && sorted_ids[j + u] == id;       // sorted: once false, false from there on
-            src[u] = mine[u] ? order[j + u] : 0;
-        }
-        Word raw[EMB_AHEAD];
-#pragma unroll
-        for (int u = 0; u < EMB_AHEAD; ++u)
-            if (mine[u]) raw[u] = *reinterpret_cast<const Word*>(d_out + static_cast<size_t>(src[u]) * C + c);
-#pragma unroll
-        for (int u = 0; u < EMB_AHEAD; ++u)
-            if (mine[u]) {
-                float f[VEC];
-                emb_unpack(raw[u], f);
-#pragma unroll
-                for (int k = 0; k < VEC; ++k) acc[k] += f[k];
+            for (int u = 0; u < EMB_AHEAD; ++u) {
+                mine[u] = j + u < n && sorted_ids[j + u] == id;       // sorted: once false, false from there on
+                src[u] = mine[u] ? order[j + u] : 0;
             }
-        if (!mine[EMB_AHEAD - 1]) break;
-    }
-    G* dst = d_table + static_cast<size_t>(id) * C + c;
-    if constexpr (sizeof(G) == 2) {
-        float o[VEC];
-        emb_unpack(*reinterpret_cast<const Word*>(dst), o);
-        alignas(16) bf16 r[VEC];
+            Word raw[EMB_AHEAD];
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) r[k] = __float2bfloat16_rn(o[k] + acc[k]);
-        *reinterpret_cast<Word*>(dst) = *reinterpret_cast<const Word*>(r);
-    } else if constexpr (VEC == 8) {
+            for (int u = 0; u < EMB_AHEAD; ++u)
+                if (mine[u]) raw[u] = *reinterpret_cast<const Word*>(d_out + static_cast<size_t>(src[u]) * C + c);
 #pragma unroll
-        for (int k = 0; k < VEC; k += 4) {
-            float4 o = *reinterpret_cast<const float4*>(dst + k);
-            o.x += acc[k]; o.y += acc[k + 1]; o.z += acc[k + 2]; o.w += acc[k + 3];
-            *reinterpret_cast<float4*>(dst + k) = o;
+            for (int u = 0; u < EMB_AHEAD; ++u)
+                if (mine[u]) {
+                    float f[VEC];
+                    emb_unpack(raw[u], f);
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) acc[k] += f[k];
+                }
+            if (!mine[EMB_AHEAD - 1]) break;
         }
-    } else {
+        G* dst = d_table + static_cast<size_t>(id) * C + c;
+        if constexpr (sizeof(G) == 2) {
+            float o[VEC];
+            emb_unpack(*reinterpret_cast<const Word*>(dst), o);
+            alignas(16) bf16 r[VEC];
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) dst[k] += acc[k];
+            for (int k = 0; k < VEC; ++k) r[k] = __float2bfloat16_rn(o[k] + acc[k]);
+            *reinterpret_cast<Word*>(dst) = *reinterpret_cast<const Word*>(r);
+        } else if constexpr (VEC == 8) {
+#pragma unroll
+            for (int k = 0; k < VEC; k += 4) {
+                float4 o = *reinterpret_cast<const float4*>(dst + k);
+                o.x += acc[k]; o.y += acc[k + 1]; o.z += acc[k + 2]; o.w += acc[k + 3];
+                *reinterpret_cast<float4*>(dst + k) = o;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) dst[k] += acc[k];
+        }
     }
 }
 
@@ -1200,7 +1202,8 @@ void embedding_bwd(const int* tokens, const void* d_out, void* d_table, int grad
 void embedding_bwd_sorted(const int* sorted_ids, const long long* order, const void* d_out, void* d_table, int grad_fp32, int n, int C, int V, int vec,
                           cudaStream_t s) {
     if (n <= 0) return;
-    const dim3 grid(n, (C + EMB_COLS - 1) / EMB_COLS);
+    const int cols = vec == 8 ? EMB_COLS : 2 * EMB_COLS;       // narrow rows: two passes of a CTA, or its launch costs more than its work
+    const dim3 grid(n, (C + cols - 1) / cols);
 #define SG_EB(G, VEC) embedding_bwd_sorted_kernel<G, VEC><<<grid, EMB_COLS / VEC, 0, s>>>(sorted_ids, order, (const bf16*)d_out, (G*)d_table, n, C, V)
     if (grad_fp32) { if (vec == 8) SG_EB(float, 8); else if (vec == 2) SG_EB(float, 2); else SG_EB(float, 1); }
     else { if (vec == 8) SG_EB(bf16, 8); else if (vec == 2) SG_EB(bf16, 2); else SG_EB(bf16, 1); }
