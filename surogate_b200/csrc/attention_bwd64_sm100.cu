@@ -14,9 +14,10 @@
 // scores of item i + 2 into the same TMEM columns.  Only MMAs of the same accumulator and shape are ordered among themselves, so the scores
 // wait for a commit of the MMA that reads P (or dS) there: X(i + 2) for dV's, while dK's runs, and Y(i + 2) for dK's (dQ's), while X(i + 2)
 // runs, so that the tensor pipe has work during both waits.  While one group computes, the other's MMAs run.  Bound by the tensor pipe: a score MMA with 64 columns re-reads its resident operand
-// from shared memory at the full 128 bytes per cycle, which makes an item 1280 (dK/dV) or 1024 (dQ) cycles; measured 1530 and 1235, where
+// from shared memory at the full 128 bytes per cycle, which makes an item 1280 (dK/dV) or 1024 (dQ) cycles; measured 1540 and 1190, where
 // one set of eight warps that took one item at a time and paid each wait, TMEM read and fence in full needed 2155 for dK/dV.
-// Both passes on B200: 2 x 4096 x 32/8 heads 1313 -> 996 us, 1 x 8192 x 40/8 2912 -> 2222 us, 8 x 2048 x 16/8 705 -> 570 us.
+// Both passes and the row statistics on B200, L2 flushed: 2 x 4096 x 32/8 heads 1312 -> 980 us, 1 x 8192 x 40/8 2906 -> 2201 us, 8 x 2048 x
+// 16/8 702 -> 562 us.
 //
 // The row statistics are laid out [B, Hq, T] beforehand (fa_delta_kernel), so that the 64 of a query tile arrive with the tile.
 // The GQA reduction of dK / dV happens in the TMEM accumulators (no atomics).  Every mbarrier wait is bounded.

@@ -872,7 +872,7 @@ static const char* launch_pair(const GemmOperand& A, const GemmOperand& B, GemmP
 // Which kernel runs a dense problem, and into how many pieces the contraction of its last wave of tiles is cut, by estimated time.  A wave
 // costs its contraction (128-byte blocks) or its epilogue, whichever is longer, and the last one both; a piece costs its trip through the
 // workspace, the warp that adds them every piece; nothing is faster than its operands and output from memory.  The constants are a
-// least-squares fit to 68 000 timings on B200 (11 500 problems, every kernel and split that they allow: profiles/gemm_kernel_choice.md);
+// least-squares fit to 68 000 timings on B200 (11 500 problems, every kernel and split that they allow);
 // blocks cost the same in bf16 and FP8.  The estimate is good to 10-20 %, so the count of pair tiles decides (a wave of them: pairs) unless
 // the other kernel is estimated 8 % faster, and a split has to promise 5 %.
 //   pair   : full rate, but 74 tiles of 256 x 256 to a wave.  [1024, 3072] = 16384 deep (48 tiles) in three pieces 164 -> 93 us, [6144, 1024] (96

@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const bf16* __r
 // out[c] = sum of the partial rows.  One CTA per 16 columns: four lanes x 16 bytes span the columns, 256 rows are read side by side, so
 // that a thread has its few loads in flight together, and the sums meet by shuffle and in shared memory (fixed order, no atomics, no
 // cleared output).  Latency-bound: a few us, where 32 CTAs whose threads walked 148 rows each, with an
-// atomic per slice and a memset before it, took 43 us for [1184, 1024].  RMSNorm backward of 16384 x 1024 on B200 83 -> 51 us in all,
-// 1024 x 512 43 -> 13 us, 8192 x 4096 90 -> 74 us.
+// atomic per slice and a memset before it, took 43 us for [1184, 1024].  RMSNorm backward on B200 in all, L2 flushed: 8192 x 4096 81 -> 65 us,
+// 3000 x 1024 53 -> 17 us, 1024 x 512 42 -> 11 us.
 constexpr int CS_COLS = 16, CS_THREADS = 1024;
 __global__ void __launch_bounds__(CS_THREADS) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int nblocks, int C) {
     __shared__ float sh[CS_THREADS / 32][CS_COLS];
@@ -937,7 +937,7 @@ constexpr float kRoundMagic = 12582912.f;   // 1.5 * 2^23: adding it rounds to t
 // reads only its own 8 elements, so the ring needs no barrier): three trips' worth of loads are outstanding while one is computed, 110 KB
 // per SM.  The group scales are two bytes each, below what cp.async moves, and are fetched one trip ahead into registers.  With loads and
 // arithmetic of a trip one after the other, DRAM idled during the arithmetic of all three CTAs: 64 M parameters in bf16
-// on B200 167 -> 141 us (4.9 TB/s).
+// on B200 170 -> 146 us (4.7 TB/s).
 // Four slots, or three where weights and gradients are both fp32: four of those leave room for two CTAs per SM only, and then the arithmetic
 // is short of warps (64 M parameters 183 us with loads and arithmetic in turn, 195 with four slots, 169 with three).
 constexpr int ADAM8_THREADS = 256;
