@@ -53,9 +53,11 @@ class Fp8Tensor:
         return Fp8Tensor(self.data.reshape(*shape), self.scale_inv, self.hp.reshape(*shape) if self.hp is not None else None)
 
     def dequantize(self) -> torch.Tensor:
-        if self.data.is_contiguous() and self.data.data_ptr() % 16 == 0 and self.scale_inv.numel() == 1:
-            return _ext().dequantize_fp8(self.data, self.scale_inv)
-        return (self.data.float() * self.scale_inv).to(torch.bfloat16)
+        q, s = self.data, self.scale_inv
+        if (q.is_cuda and s.is_cuda and q.dtype in (torch.float8_e4m3fn, torch.float8_e5m2) and s.dtype == torch.float32 and s.numel() == 1
+                and q.is_contiguous() and q.data_ptr() % 16 == 0):
+            return _ext().dequantize_fp8(q, s)
+        return (q.float() * s).to(torch.bfloat16)
 
 
 def gemm(a, b, out=None, *, a_mn=False, b_mn=False, accumulate=False, alpha=1.0, scale_a=None, scale_b=None, amax_out=None,
