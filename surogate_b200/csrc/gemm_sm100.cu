@@ -175,11 +175,12 @@ struct Unit {
     int tile, kb0, kb1;
     int piece;   // -1: a whole tile
 };
-__device__ __forceinline__ int num_units(const GemmParams& p, int num_tiles) {
-    return p.splits > 1 ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
+// Kernels for whole problems (SPLIT = false) are instantiations of their own: the code of the pieces costs registers and 0.1-0.3 us of a short launch.
+template <bool SPLIT> __device__ __forceinline__ int num_units(const GemmParams& p, int num_tiles) {
+    return SPLIT ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
 }
-__device__ __forceinline__ Unit get_unit(const GemmParams& p, int num_tiles, int num_k, int unit) {
-    if (p.splits <= 1 || unit < p.split_from) return Unit{unit, 0, num_k, -1};
+template <bool SPLIT> __device__ __forceinline__ Unit get_unit(const GemmParams& p, int num_tiles, int num_k, int unit) {
+    if (!SPLIT || unit < p.split_from) return Unit{unit, 0, num_k, -1};
     const int r = unit - p.split_from, n = num_tiles - p.split_from;
     const int s = r / n;
     return Unit{p.split_from + r % n, s * num_k / p.splits, (s + 1) * num_k / p.splits, s};
@@ -233,7 +234,7 @@ __device__ __forceinline__ bool last_piece(int* counter, int pieces, int lane) {
     return true;
 }
 
-template <int BN>
+template <int BN, bool SPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
     using C = Cfg<BN>;
@@ -293,7 +294,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
     const int num_tiles = num_tiles_sh;
-    const int units = num_units(p, num_tiles);      // grouped problems are never split: a unit is a tile
+    const int units = num_units<SPLIT>(p, num_tiles);      // grouped problems are never split: a unit is a tile
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -305,10 +306,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int chunk_bytes = BK * TILE_K_BYTES;   // MN-major chunk: BK rows of 128 B
             bool ok = true;
             for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
-                const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
+                const Unit u = get_unit<SPLIT>(p, num_tiles, (p.K + BK - 1) / BK, unit);
                 const TileInfo t = get_tile<BN>(p, tile_start, u.tile, BK);
                 const int m0 = t.a_row0, n0 = t.b_row0;
-                const int kb1 = u.piece < 0 ? t.num_k : u.kb1;
+                const int kb1 = !SPLIT || u.piece < 0 ? t.num_k : u.kb1;
                 for (int kb = u.kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, &abort_flag)) { ok = false; break; }
                     const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
@@ -347,8 +348,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 acc_phase[acc] ^= 1u;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
-                const int num_k = u.piece < 0 ? get_tile<BN>(p, tile_start, u.tile, BK).num_k : u.kb1 - u.kb0;
+                const Unit u = get_unit<SPLIT>(p, num_tiles, (p.K + BK - 1) / BK, unit);
+                const int num_k = !SPLIT || u.piece < 0 ? get_tile<BN>(p, tile_start, u.tile, BK).num_k : u.kb1 - u.kb0;
                 for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, &abort_flag)) { ok = false; break; }
                     tc_fence_after();
@@ -379,7 +380,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         float amax = 0.f;
         bool ok = true;
         for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local_tile) {
-            const Unit u = get_unit(p, num_tiles, (p.K + BK - 1) / BK, unit);
+            const Unit u = get_unit<SPLIT>(p, num_tiles, (p.K + BK - 1) / BK, unit);
             const TileInfo t = get_tile<BN>(p, tile_start, u.tile, BK);
             const int acc = local_tile & 1;
             if (!mbar_wait(tfull_bar(acc), acc_phase[acc], &abort_flag)) { ok = false; break; }
@@ -387,7 +388,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             tc_fence_after();
             const int row = t.d_row0 + quad * 32 + lane;
             const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-            if (u.piece >= 0) {
+            if (SPLIT && u.piece >= 0) {
                 const int slot = (u.tile - p.split_from) * 4 + quad, slots = (num_tiles - p.split_from) * 4;
                 float4* ws = reinterpret_cast<float4*>(p.workspace) + static_cast<size_t>(slot) * (32 * BN / 4);
                 const size_t stride = static_cast<size_t>(slots) * (32 * BN / 4);
@@ -468,7 +469,7 @@ __device__ __forceinline__ PairTile pair_tile(const GemmParams& p, int tile) {
     return PairTile{(first_m + r % gsize) * PAIR_BM, (r / gsize) * PAIR_BN};
 }
 
-template <bool ACC>
+template <bool ACC, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmD,
                  const GemmParams p, const int use_tma_store) {
@@ -493,7 +494,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int BK = TILE_K_BYTES / p.elem_bytes;
     const int num_tiles = ((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
     const int num_k = (p.K + BK - 1) / BK;
-    const int units = num_units(p, num_tiles);
+    const int units = num_units<SPLIT>(p, num_tiles);
     const int first_unit = blockIdx.x >> 1, unit_step = gridDim.x >> 1;
 
     if (threadIdx.x == 0) {
@@ -534,7 +535,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // optional L2 prefetch cursor: runs `pair_prefetch` contraction blocks ahead of the load cursor (across tile boundaries)
             int pf_unit = first_unit, pf_kb = 0, pf_end = 0, pf_m0 = 0, pf_n0 = 0;
             auto pf_origin = [&]() {
-                const Unit u = get_unit(p, num_tiles, num_k, pf_unit);
+                const Unit u = get_unit<SPLIT>(p, num_tiles, num_k, pf_unit);
                 const PairTile t = pair_tile(p, u.tile);
                 pf_kb = u.kb0;
                 pf_end = u.kb1;
@@ -558,7 +559,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 for (int i = 0; i < PAIR_STAGES + p.pair_prefetch; ++i) pf_step();
             }
             for (int unit = first_unit; unit < units && ok; unit += unit_step) {
-                const Unit u = get_unit(p, num_tiles, num_k, unit);
+                const Unit u = get_unit<SPLIT>(p, num_tiles, num_k, unit);
                 const PairTile t = pair_tile(p, u.tile);
                 const int m0 = t.m0 + static_cast<int>(rank) * 128, n0 = t.n0 + static_cast<int>(rank) * 128;
                 for (int kb = u.kb0; kb < u.kb1; ++kb) {
@@ -601,7 +602,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 acc_phase[acc] ^= 1u;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
-                const Unit u = get_unit(p, num_tiles, num_k, unit);
+                const Unit u = get_unit<SPLIT>(p, num_tiles, num_k, unit);
                 for (int kb = 0; kb < u.kb1 - u.kb0; ++kb) {
                     if (!mbar_wait_cluster(full_bar(stage), phase, &abort_flag)) { ok = false; break; }
                     tc_fence_after();
@@ -724,16 +725,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
         };
         for (int unit = first_unit; unit < units && ok; unit += unit_step, ++local_tile) {
-            const Unit u = get_unit(p, num_tiles, num_k, unit);
+            const Unit u = get_unit<SPLIT>(p, num_tiles, num_k, unit);
             const PairTile pt = pair_tile(p, u.tile);
             const int acc = local_tile & 1;
             const int row_w = pt.m0 + static_cast<int>(rank) * 128 + quad * 32;   // first row of this warp
             const uint32_t t_row = tmem_base + acc * PAIR_BN + (static_cast<uint32_t>(quad * 32) << 16);
-            if (u.piece < 0) fetch_d(pt, row_w);
+            if (!SPLIT || u.piece < 0) fetch_d(pt, row_w);
             if (!mbar_wait(tfull_bar(acc), acc_phase[acc], &abort_flag)) { ok = false; break; }
             acc_phase[acc] ^= 1u;
             tc_fence_after();
-            if (u.piece < 0) {
+            if (!SPLIT || u.piece < 0) {
                 emit(pt, row_w, [&](int c, uint32_t(&r)[32]) { tmem_ld_32x32(t_row + c, r); });
                 tc_fence_before();
                 __syncwarp();
@@ -802,7 +803,7 @@ const char* make_tensor_map_2d(CUtensorMap* map, const void* base, int elem_byte
     return r == CUDA_SUCCESS ? nullptr : "cuTensorMapEncodeTiled failed";
 }
 
-template <int BN> static const char* launch(const GemmOperand& A, const GemmOperand& B, const GemmParams& p, int num_sms, cudaStream_t stream) {
+template <int BN, bool SPLIT> static const char* launch(const GemmOperand& A, const GemmOperand& B, const GemmParams& p, int num_sms, cudaStream_t stream) {
     using C = Cfg<BN>;
     const int BK = TILE_K_BYTES / p.elem_bytes;
     CUtensorMap tmA, tmB;
@@ -818,11 +819,11 @@ template <int BN> static const char* launch(const GemmOperand& A, const GemmOper
     else e = make_tensor_map_2d(&tmB, B.ptr, p.elem_bytes, p.N, b_rows, B.row_stride_bytes, BK, BK);
     if (e) return e;
     static std::atomic<uint64_t> limit{0};
-    if (!raise_smem_limit(reinterpret_cast<const void*>(gemm_tcgen05_kernel<BN>), C::SMEM_BYTES, limit)) return "raising the shared-memory limit failed (GEMM)";
+    if (!raise_smem_limit(reinterpret_cast<const void*>(gemm_tcgen05_kernel<BN, SPLIT>), C::SMEM_BYTES, limit)) return "raising the shared-memory limit failed (GEMM)";
     int units = p.mode == 0 ? ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) : num_sms;  // grouped: tile count lives on the device
-    if (p.splits > 1) units = p.split_from + (units - p.split_from) * p.splits;
+    if (SPLIT) units = p.split_from + (units - p.split_from) * p.splits;
     const int grid = units < num_sms ? units : num_sms;
-    gemm_tcgen05_kernel<BN><<<grid, GEMM_THREADS, C::SMEM_BYTES, stream>>>(tmA, tmB, p);
+    gemm_tcgen05_kernel<BN, SPLIT><<<grid, GEMM_THREADS, C::SMEM_BYTES, stream>>>(tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? nullptr : "gemm kernel launch failed";
 }
 
@@ -856,16 +857,17 @@ static const char* launch_pair(const GemmOperand& A, const GemmOperand& B, GemmP
     }
     if (!use_tma_store) tmD = tmA;
     const bool acc = use_tma_store && p.accumulate && !p.out_fp32;
-    static std::atomic<uint64_t> limit[2];
-    if (!(acc ? raise_smem_limit(reinterpret_cast<const void*>(gemm_pair_kernel<true>), PairCfg<true>::SMEM_BYTES, limit[1])
-              : raise_smem_limit(reinterpret_cast<const void*>(gemm_pair_kernel<false>), PairCfg<false>::SMEM_BYTES, limit[0])))
-        return "raising the shared-memory limit failed (pair GEMM)";
     const int num_tiles = ((p.M + PAIR_BM - 1) / PAIR_BM) * ((p.N + PAIR_BN - 1) / PAIR_BN);
     const int units = p.splits > 1 ? p.split_from + (num_tiles - p.split_from) * p.splits : num_tiles;
     const int clusters = units < num_sms / 2 ? units : num_sms / 2;
-    if (acc) gemm_pair_kernel<true><<<2 * clusters, GEMM_THREADS, PairCfg<true>::SMEM_BYTES, stream>>>(tmA, tmB, tmD, p, use_tma_store);
-    else gemm_pair_kernel<false><<<2 * clusters, GEMM_THREADS, PairCfg<false>::SMEM_BYTES, stream>>>(tmA, tmB, tmD, p, use_tma_store);
-    return cudaGetLastError() == cudaSuccess ? nullptr : "pair gemm kernel launch failed";
+    auto run = [&](auto* kernel, int smem, std::atomic<uint64_t>& limit) -> const char* {
+        if (!raise_smem_limit(reinterpret_cast<const void*>(kernel), smem, limit)) return "raising the shared-memory limit failed (pair GEMM)";
+        kernel<<<2 * clusters, GEMM_THREADS, smem, stream>>>(tmA, tmB, tmD, p, use_tma_store);
+        return cudaGetLastError() == cudaSuccess ? nullptr : "pair gemm kernel launch failed";
+    };
+    static std::atomic<uint64_t> limit[4];
+    if (acc) return p.splits > 1 ? run(gemm_pair_kernel<true, true>, PairCfg<true>::SMEM_BYTES, limit[3]) : run(gemm_pair_kernel<true, false>, PairCfg<true>::SMEM_BYTES, limit[2]);
+    return p.splits > 1 ? run(gemm_pair_kernel<false, true>, PairCfg<false>::SMEM_BYTES, limit[1]) : run(gemm_pair_kernel<false, false>, PairCfg<false>::SMEM_BYTES, limit[0]);
 }
 
 // ------------------------------------------------------------------------------------------------ choice of kernel and split
@@ -958,7 +960,8 @@ const char* gemm_sm100(const GemmOperand& A, const GemmOperand& B, GemmParams p,
     // 128-wide N tiles when the wide tile would leave SMs idle or N is small
     const long tiles256 = static_cast<long>((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
     const bool narrow = p.mode == 0 ? p.tile_n != 256 : p.N <= 128 || (p.tile_n == 128) || (p.tile_n == 0 && tiles256 < num_sms);
-    return narrow ? launch<128>(A, B, p, num_sms, stream) : launch<256>(A, B, p, num_sms, stream);
+    if (p.splits > 1) return launch<128, true>(A, B, p, num_sms, stream);      // only the narrow tiles are ever cut
+    return narrow ? launch<128, false>(A, B, p, num_sms, stream) : launch<256, false>(A, B, p, num_sms, stream);
 }
 
 }  // namespace sg
