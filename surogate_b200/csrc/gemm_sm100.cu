@@ -921,13 +921,14 @@ GemmPlan gemm_plan_sm100(const GemmParams& p, int num_sms) {
     constexpr float pair_out[4] = {4.0f, 5.4f, 5.2f, 5.8f}, single_out[4] = {3.7f, 7.7f, 5.3f, 13.0f}, single_block[3] = {0.26f, 0.27f, 0.32f};
     const Shape pair{up(p.M, PAIR_BM) * up(p.N, PAIR_BN), num_sms / 2, 1.6f, 0.41f, pair_out[out], 7.2f, 1.2f, 1.5f, PAIR_BM * PAIR_BN};
     // operands of fewer than 16 rows, or with stored rows below 32 bytes, arrive slowly: 2-5 us more per piece
-    const bool thin = p.M < 16 || (p.a_mn && p.M * p.elem_bytes < 32) || (p.b_mn && p.N * p.elem_bytes < 32);
-    const float single_piece = thin ? 11.3f : 6.3f;
+    const bool short_rows = (p.a_mn && p.M * p.elem_bytes < 32) || (p.b_mn && p.N * p.elem_bytes < 32);
+    const float single_piece = p.M < 16 || short_rows ? 11.3f : 6.3f;
     const Shape single{up(p.M, BM) * up(p.N, 128), num_sms, 0.4f, single_block[mn], single_out[out], single_piece, 0.4f, 0.4f, BM * 128};
     const float stream_us = (static_cast<float>(p.elem_bytes) * p.K * (static_cast<float>(p.M) + p.N) +
                              (p.out_fp32 ? 4.f : 2.f) * (p.accumulate ? 2.f : 1.f) * p.M * p.N) / STREAM_BYTES_PER_US;
     const Split sp = best_split(pair, num_k, stream_us), ss = best_split(single, num_k, stream_us);
-    int use_pair = p.N > 128 && (pair.tiles >= pair.slots ? !(ss.us < KERNEL_GAIN * sp.us) : sp.us < KERNEL_GAIN * ss.us);
+    // stored rows below 32 bytes slow single CTAs more than pairs, beyond the estimate: 16 x 151936 in FP8, 512 deep, 98 and 78 us
+    int use_pair = p.N > 128 && (pair.tiles >= pair.slots ? short_rows || !(ss.us < KERNEL_GAIN * sp.us) : sp.us < KERNEL_GAIN * ss.us);
     if (p.tile_n != 0) use_pair = p.tile_n == 512;
     plan.pair = use_pair;
     if (p.tile_n == 256 || p.tile_n == 128) return plan;        // forced single-CTA tiles: never split

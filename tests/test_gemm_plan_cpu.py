@@ -29,6 +29,7 @@ def plan():
     (dict(M=1, N=4096, K=12288), False, True),                                 # whole 58 -> 31
     (dict(M=8192, N=16, K=8192, elem=1, b_mn=True), False, False),             # two pieces 27 -> 25
     (dict(M=16, N=6144, K=8192, elem=1, a_mn=True, b_mn=True), False, False),  # three pieces 27 -> 24
+    (dict(M=16, N=151936, K=512, elem=1, a_mn=True, b_mn=True), True, False),  # single CTAs 98 -> 78
     (dict(M=6144, N=1024, K=16384, a_mn=True, b_mn=True), True, True),         # whole 204 -> 157
     (dict(M=4096, N=16, K=17408, b_mn=True), False, True),                     # whole 91 -> 45
     (dict(M=8192, N=4096, K=4096), True, False),
